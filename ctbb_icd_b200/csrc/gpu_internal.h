@@ -51,6 +51,14 @@ struct ctbb_ctx {
 // first entry of SSM view v, so a view window [v0, v1) is one contiguous run.
 struct ctbb_ssm {
     ctbb_ctx* ctx = nullptr;
+    // Unique for the life of the process: what a reconstruction keeps about a
+    // matrix (captured launches, entry counts) is keyed by it, since a later
+    // matrix may be allocated at the same addresses.
+    uint64_t id = next_id();
+    static uint64_t next_id() {
+        static std::atomic<uint64_t> n{0};
+        return ++n;
+    }
     ctbb_geom_c geom{};
     uint64_t ncol = 0, nvsm = 0, nnz = 0, max_col_nnz = 0;
     int64_t* d_colptr = nullptr;  // [ncol + 1]
@@ -88,7 +96,7 @@ struct ctbb_recon {
     float* d_e32 = nullptr;      // grouped-mode y - A x
     int rep = 0;                 // 0: x64/est64 current, 1: x32/e32 current
     // Sum over voxels inside the FOV of in-range matrix entries (cached per matrix).
-    const ctbb_ssm* entries_ssm = nullptr;
+    uint64_t entries_ssm = 0;
     double entries = 0.0;
     // Grouped-mode visiting order: packed (column * nz + slice) per item,
     // built once per lattice spacing.

@@ -2067,6 +2067,7 @@ ctbb_status launch_staged(const GParams& P, const uint32_t* order, const ctbb_ss
 // unchanged (byte comparison; the struct is zero-filled before use).
 struct GraphKey {
     GParams P;
+    uint64_t ssm;  // the matrix (its id, not its address)
     const void* order;
     const void* stacks;
     const void* w;
@@ -2099,7 +2100,7 @@ ctbb_status build_order(ctbb_recon* rc, int P_lat) {
 namespace ctbb {
 
 ctbb_status inrange_entries(ctbb_recon* rc, const ctbb_ssm* ssm, double* out) {
-    if (rc->entries_ssm != ssm) {
+    if (rc->entries_ssm != ssm->id) {
         ctbb_icd_opts o{};
         const GParams P = make_params(rc, ssm, o);
         ctbb_ctx* ctx = rc->ctx;
@@ -2111,7 +2112,7 @@ ctbb_status inrange_entries(ctbb_recon* rc, const ctbb_ssm* ssm, double* out) {
         CTBB_CUDA(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
         CTBB_CUDA(cudaStreamSynchronize(ctx->stream));
         rc->entries = (double)h;
-        rc->entries_ssm = ssm;
+        rc->entries_ssm = ssm->id;
     }
     *out = rc->entries;
     return CTBB_OK;
@@ -2340,6 +2341,7 @@ ctbb_status launch_icd_grouped(ctbb_recon* rc, const ctbb_ssm* ssm, const ctbb_i
     GraphKey key;
     memset(&key, 0, sizeof(key));
     key.P = P;
+    key.ssm = ssm->id;
     key.order = order;
     key.stacks = stacks;
     key.w = pairs ? (const void*)ssm->d_pairs : h ? (const void*)ssm->d_w16 : (const void*)ssm->d_w32;
