@@ -220,12 +220,17 @@ __global__ void __launch_bounds__(256) conv_mid_kernel(Dims d, const __nv_bfloat
 // Weight gradient of a C -> C convolution (tensor cores):
 //   dW[t][ci][co] += sum_v X[v + off(t)][ci] * dY[v][co].
 // Work unit u = (tap t = u / 2, ci half u % 2); warp w owns units w, w+8, ...
-// Per-CTA FP32 partials are added to dw with atomics once at the end.
-constexpr int kUnitsPerWarp = 7;  // ceil(54 / 8)
+// Unit 54 (a free slot of warp 6) multiplies dY by a matrix of ones: its rows
+// are the bias gradient db[co] += sum_v dY[v][co], so dY needs no second pass
+// (a kernel of its own took 117 us per layer at 8 x 128 x 128).
+// Per-CTA FP32 partials are added to dw and db with atomics once at the end.
+constexpr int kUnitsPerWarp = 7;  // ceil(55 / 8)
+constexpr int kBiasUnit = 2 * kTaps;
+constexpr uint32_t kOnes = 0x3F803F80u;  // two BF16 ones
 
 __global__ void __launch_bounds__(256) conv_wgrad_kernel(Dims d, const __nv_bfloat16* __restrict__ x,
                                                          const __nv_bfloat16* __restrict__ dy,
-                                                         float* __restrict__ dw) {
+                                                         float* __restrict__ dw, float* __restrict__ db) {
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t s_halo = (uint32_t)__cvta_generic_to_shared(smem);
     const uint32_t s_dy = s_halo + kHalo * kRowBytes;
@@ -276,6 +281,18 @@ __global__ void __launch_bounds__(256) conv_wgrad_kernel(Dims d, const __nv_bflo
 #pragma unroll
                 for (int n = 0; n < 4; ++n) mma_bf16(acc[u][n], a0, a1, a2, a3, b[n][0], b[n][1]);
             }
+            if (warp == kBiasUnit % 8) {
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+                    mma_bf16(acc[kBiasUnit / 8][n], kOnes, kOnes, kOnes, kOnes, b[n][0], b[n][1]);
+            }
+        }
+    }
+    if (warp == kBiasUnit % 8 && lane < 4) {  // row 0 of the product
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            atomicAdd(db + n * 8 + lane * 2, acc[kBiasUnit / 8][n][0]);
+            atomicAdd(db + n * 8 + lane * 2 + 1, acc[kBiasUnit / 8][n][1]);
         }
     }
 #pragma unroll
@@ -428,70 +445,118 @@ __global__ void __launch_bounds__(256) conv_out_bwd_kernel(int nx, int ny, int n
     }
 }
 
-// Weight gradients of the 1-channel layers. Thread (tq, c) of a 288-thread
-// block owns taps tq, tq + 9, tq + 18 of channel c and sums over a chunk of
-// voxels; per-block sums go to dw with atomics.
+// Weight gradients of the 1-channel layers:
 //   mode 0 (conv_out): dw[t][c] += sum_v a[v + off(t)][c] * dout[v];  dw[27*32] += sum dout
 //   mode 1 (conv_in):  dw[t][c] += sum_v s_in x[v + off(t)] * g[v][c] * (a0[v][c] > 0);
 //                      dw[27*32 + c] += sum_v g[v][c] * (a0[v][c] > 0)
-constexpr int kWg1Threads = 288;
-constexpr int kWg1Chunk = 1024;
+// Both are outer products per voxel of its 32 activations with the 27
+// neighbours of a scalar field (mode 0 after shifting the sum by off(t), which
+// mirrors the taps). Lane c of a warp holds channel c's 27 sums in registers and
+// walks a row of voxels; the field's halo of a 32 x 8 tile is in shared memory,
+// and the 3 x 3 x 3 window slides along x, so a voxel costs one coalesced
+// 64-byte load, 9 shared-memory broadcasts and 27 FMAs. Bound by issue and the
+// shared-memory reads. (One thread per tap triple and channel walking 1024
+// voxels serially, three dependent global loads each, took 900 us per launch at
+// 8 x 128 x 128.)
+constexpr int kW1X = 32, kW1Y = 8;
+constexpr int kW1PerSm = 4;  // persistent blocks per SM
+constexpr int kW1HX = kW1X + 2, kW1HY = kW1Y + 2;
 
-__global__ void __launch_bounds__(kWg1Threads) wgrad_1ch_kernel(int mode, int nx, int ny, int nz,
-                                                                 const __nv_bfloat16* __restrict__ act,
-                                                                 const float* __restrict__ scal, float s_in,
-                                                                 const __nv_bfloat16* __restrict__ mask,
-                                                                 float* __restrict__ dw) {
-    const int c = threadIdx.x & 31, tq = threadIdx.x >> 5;
-    const uint64_t n = (uint64_t)nx * ny * nz;
-    float acc[3] = {0.f, 0.f, 0.f};
+template <int MODE>
+__global__ void __launch_bounds__(256) wgrad_1ch_kernel(int nx, int ny, int nz, int tiles_x, int tiles_y,
+                                                        uint64_t n_tiles, const __nv_bfloat16* __restrict__ act,
+                                                        const float* __restrict__ scal, float s_in,
+                                                        const __nv_bfloat16* __restrict__ mask,
+                                                        float* __restrict__ part) {
+    __shared__ float sh[3 * kW1HY * kW1HX];
+    __shared__ float red[8][(kTaps + 1) * kC];
+    const int c = threadIdx.x & 31, row = threadIdx.x >> 5;
+    float acc[kTaps];
+#pragma unroll
+    for (int t = 0; t < kTaps; ++t) acc[t] = 0.f;
     float accb = 0.f;
-    const uint64_t v0 = (uint64_t)blockIdx.x * kWg1Chunk;
-    const uint64_t v1 = min(n, v0 + kWg1Chunk);
-    for (uint64_t v = v0; v < v1; ++v) {
-        const int ix = (int)(v % nx), iy = (int)((v / nx) % ny), iz = (int)(v / ((uint64_t)nx * ny));
-        if (mode == 0) {
-            const float dv = scal[v];
-            if (tq == 0 && c == 0) accb += dv;
+    for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+        const int x0 = (int)(tile % tiles_x) * kW1X;
+        const uint64_t r = tile / tiles_x;
+        const int y0 = (int)(r % tiles_y) * kW1Y, z = (int)(r / tiles_y);
+        __syncthreads();  // previous tile's halo fully read
+        for (int i = threadIdx.x; i < 3 * kW1HY * kW1HX; i += blockDim.x) {
+            const int jx = x0 + i % kW1HX - 1, jy = y0 + (i / kW1HX) % kW1HY - 1, jz = z + i / (kW1HX * kW1HY) - 1;
+            sh[i] = inside(jx, jy, jz, nx, ny, nz)
+                        ? (MODE == 1 ? s_in : 1.f) * scal[((uint64_t)jz * ny + jy) * nx + jx]
+                        : 0.f;
+        }
+        __syncthreads();
+        const int y = y0 + row;
+        if (y >= ny) continue;
+        const int nxt = min(kW1X, nx - x0);
+        const uint64_t v0 = ((uint64_t)z * ny + y) * nx + x0;
+        // win[q][m]: line q = dz * 3 + dy of the window, column m (mod 3).
+        float win[9][3];
+        const float* line[3];
 #pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                const int t = tq + 9 * q;
-                const int jx = ix + t % 3 - 1, jy = iy + (t / 3) % 3 - 1, jz = iz + t / 9 - 1;
-                if (!inside(jx, jy, jz, nx, ny, nz)) continue;
-                acc[q] = fmaf(__bfloat162float(act[(((uint64_t)jz * ny + jy) * nx + jx) * kC + c]), dv, acc[q]);
+        for (int dz = 0; dz < 3; ++dz) {
+            line[dz] = sh + (dz * kW1HY + row) * kW1HX;
+#pragma unroll
+            for (int dy = 0; dy < 3; ++dy) {
+                win[dz * 3 + dy][0] = line[dz][dy * kW1HX];
+                win[dz * 3 + dy][1] = line[dz][dy * kW1HX + 1];
             }
-        } else {
-            float gv = __bfloat162float(act[v * kC + c]);
-            if (!(__bfloat162float(mask[v * kC + c]) > 0.f)) gv = 0.f;
-            if (tq == 0) accb += gv;
+        }
+        auto value = [&](int x) {
+            float v = __bfloat162float(act[(v0 + x) * kC + c]);
+            if (MODE == 1 && !(__bfloat162float(mask[(v0 + x) * kC + c]) > 0.f)) v = 0.f;
+            return v;
+        };
+        for (int xb = 0; xb < kW1X; xb += 3) {
+            float a[3];
 #pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                const int t = tq + 9 * q;
-                const int jx = ix + t % 3 - 1, jy = iy + (t / 3) % 3 - 1, jz = iz + t / 9 - 1;
-                if (!inside(jx, jy, jz, nx, ny, nz)) continue;
-                acc[q] = fmaf(s_in * scal[((uint64_t)jz * ny + jy) * nx + jx], gv, acc[q]);
+            for (int u = 0; u < 3; ++u) a[u] = xb + u < nxt ? value(xb + u) : 0.f;
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                const int x = xb + u;
+                if (x >= nxt) break;  // uniform in the warp
+#pragma unroll
+                for (int q = 0; q < 9; ++q) win[q][(u + 2) % 3] = line[q / 3][(q % 3) * kW1HX + x + 2];
+#pragma unroll
+                for (int q = 0; q < 9; ++q)
+#pragma unroll
+                    for (int dx = 0; dx < 3; ++dx)
+                        acc[q * 3 + dx] = fmaf(a[u], win[q][(u + dx) % 3], acc[q * 3 + dx]);
+                accb += MODE == 1 ? a[u] : win[4][(u + 1) % 3];
             }
         }
     }
+    // The block's eight warps summed in a fixed order; blocks are summed in
+    // order by wgrad_1ch_sum_kernel, so the gradient is reproducible.
 #pragma unroll
-    for (int q = 0; q < 3; ++q) atomicAdd(dw + (tq + 9 * q) * kC + c, acc[q]);
-    if (mode == 0 && tq == 0 && c == 0) atomicAdd(dw + kTaps * kC, accb);
-    if (mode == 1 && tq == 0) atomicAdd(dw + kTaps * kC + c, accb);
+    for (int t = 0; t < kTaps; ++t) red[row][t * kC + c] = acc[t];
+    red[row][kTaps * kC + c] = accb;
+    __syncthreads();
+    for (int i = threadIdx.x; i < (kTaps + 1) * kC; i += blockDim.x) {
+        float v = red[0][i];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) v += red[w][i];
+        part[(uint64_t)blockIdx.x * (kTaps + 1) * kC + i] = v;
+    }
 }
 
-// db[c] += sum_v dy[v][c].
-__global__ void __launch_bounds__(256) bias_grad_kernel(uint64_t n, const __nv_bfloat16* __restrict__ dy,
-                                                        float* __restrict__ db) {
+// dw += the blocks' partial sums, one block of 256 threads per tap (27: the bias).
+template <int MODE>
+__global__ void __launch_bounds__(256) wgrad_1ch_sum_kernel(int n_blocks, const float* __restrict__ part,
+                                                            float* __restrict__ dw) {
     __shared__ float sh[8][kC];
-    const int c = threadIdx.x & 31, r = threadIdx.x >> 5;
+    const int t = blockIdx.x, c = threadIdx.x & 31, g = threadIdx.x >> 5;
     float s = 0.f;
-    for (uint64_t v = blockIdx.x * 8ull + r; v < n; v += gridDim.x * 8ull) s += __bfloat162float(dy[v * kC + c]);
-    sh[r][c] = s;
+    for (int b = g; b < n_blocks; b += 8) s += part[((uint64_t)b * (kTaps + 1) + t) * kC + c];
+    sh[g][c] = s;
     __syncthreads();
-    if (r == 0) {
-        for (int i = 1; i < 8; ++i) s += sh[i][c];
-        atomicAdd(db + c, s);
-    }
+    if (g) return;
+    for (int i = 1; i < 8; ++i) s += sh[i][c];
+    if (t < kTaps)
+        dw[(MODE == 0 ? kTaps - 1 - t : t) * kC + c] += s;
+    else if (MODE == 1 || c == 0)  // mode 0: every lane holds the same sum of dout
+        dw[kTaps * kC + c] += s;
 }
 
 __global__ void adam_kernel(uint64_t n, float* __restrict__ p, float* __restrict__ g, float* __restrict__ m,
@@ -570,6 +635,7 @@ struct ctbb_cnn {
     __nv_bfloat16* d_act = nullptr;
     float* d_out = nullptr;
     float* d_dout = nullptr;
+    float* d_wpart = nullptr;  // per-block partial gradients of the one-channel layers
     __nv_bfloat16* a(int l) { return d_act + (uint64_t)l * cap * kC; }
     __nv_bfloat16* h(int l) { return d_act + (uint64_t)(blocks + 1 + l) * cap * kC; }
     __nv_bfloat16* gbuf(int i) { return d_act + (uint64_t)(2 * blocks + 1 + i) * cap * kC; }
@@ -648,10 +714,11 @@ ctbb_status check_conv_flag(ctbb_cnn* c) {
     return CTBB_OK;
 }
 
-ctbb_status conv_wgrad(ctbb_cnn* c, const Dims& d, const __nv_bfloat16* x, const __nv_bfloat16* dy, float* dw) {
+ctbb_status conv_wgrad(ctbb_cnn* c, const Dims& d, const __nv_bfloat16* x, const __nv_bfloat16* dy, float* dw,
+                       float* db) {
     CTBB_TRY(configure_kernels(c->ctx->device));
     const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(d.n_tiles, (uint64_t)c->ctx->sm_count * 2));
-    conv_wgrad_kernel<<<grid, 256, kWgSmem, c->ctx->stream>>>(d, x, dy, dw);
+    conv_wgrad_kernel<<<grid, 256, kWgSmem, c->ctx->stream>>>(d, x, dy, dw, db);
     CTBB_CUDA(cudaGetLastError());
     return CTBB_OK;
 }
@@ -739,6 +806,7 @@ extern "C" ctbb_status ctbb_cnn_create(ctbb_ctx* ctx, int32_t blocks, uint64_t s
     CTBB_CUDA(cudaMalloc(&c->d_m, o * sizeof(float)));
     CTBB_CUDA(cudaMalloc(&c->d_v, o * sizeof(float)));
     const size_t nw = std::max<size_t>(1, (size_t)2 * blocks) * kConvW;
+    CTBB_CUDA(cudaMalloc(&c->d_wpart, (size_t)ctx->sm_count * kW1PerSm * (kTaps + 1) * kC * sizeof(float)));
     CTBB_CUDA(cudaMalloc(&c->d_wf, nw * sizeof(__nv_bfloat16)));
     CTBB_CUDA(cudaMalloc(&c->d_wb, nw * sizeof(__nv_bfloat16)));
     CTBB_CUDA(cudaMalloc(&c->d_offs, std::max<size_t>(1, c->off_w.size()) * sizeof(uint64_t)));
@@ -766,6 +834,7 @@ extern "C" void ctbb_cnn_free(ctbb_cnn* c) {
     cudaFree(c->d_g);
     cudaFree(c->d_m);
     cudaFree(c->d_v);
+    cudaFree(c->d_wpart);
     cudaFree(c->d_wf);
     cudaFree(c->d_wb);
     cudaFree(c->d_offs);
@@ -866,9 +935,13 @@ extern "C" ctbb_status ctbb_cnn_accumulate_gradient(ctbb_cnn* c, const float* x_
     CTBB_TRY(reduce(ctx, lg, &L));
     const int B = c->blocks;
     // out = conv_out(a_B) + b_out
-    const int wg_blocks = (int)((n + kWg1Chunk - 1) / kWg1Chunk);
-    wgrad_1ch_kernel<<<wg_blocks, kWg1Threads, 0, st>>>(0, nx, ny, nz, c->a(B), c->d_dout, 0.f, nullptr,
-                                                         c->d_g + c->off_wout);
+    const int w1x = (nx + kW1X - 1) / kW1X, w1y = (ny + kW1Y - 1) / kW1Y;
+    const uint64_t w1tiles = (uint64_t)w1x * w1y * nz;
+    const int wg_blocks = (int)std::min<uint64_t>(w1tiles, (uint64_t)ctx->sm_count * kW1PerSm);
+    wgrad_1ch_kernel<0><<<wg_blocks, 256, 0, st>>>(nx, ny, nz, w1x, w1y, w1tiles, c->a(B), c->d_dout, 0.f, nullptr,
+                                                   c->d_wpart);
+    CTBB_CUDA(cudaGetLastError());
+    wgrad_1ch_sum_kernel<0><<<kTaps + 1, 256, 0, st>>>(wg_blocks, c->d_wpart, c->d_g + c->off_wout);
     CTBB_CUDA(cudaGetLastError());
     conv_out_bwd_kernel<<<grid1(ctx, n), 256, 0, st>>>(nx, ny, nz, c->d_dout, c->d_p + c->off_wout, c->gbuf(0));
     CTBB_CUDA(cudaGetLastError());
@@ -876,21 +949,19 @@ extern "C" ctbb_status ctbb_cnn_accumulate_gradient(ctbb_cnn* c, const float* x_
     for (int l = B - 1; l >= 0; --l) {
         __nv_bfloat16* g = c->gbuf(gi);
         // a_{l+1} = a_l + conv(h_l; W2) + b2
-        CTBB_TRY(conv_wgrad(c, d, c->h(l), g, c->d_g + c->off_w[2 * l + 1]));
-        bias_grad_kernel<<<grid1(ctx, n / 8 + 1), 256, 0, st>>>(n, g, c->d_g + c->off_b[2 * l + 1]);
-        CTBB_CUDA(cudaGetLastError());
+        CTBB_TRY(conv_wgrad(c, d, c->h(l), g, c->d_g + c->off_w[2 * l + 1], c->d_g + c->off_b[2 * l + 1]));
         CTBB_TRY(conv_mid(c, d, g, c->d_wb + (uint64_t)(2 * l + 1) * kConvW, nullptr, nullptr, c->h(l), 0, c->du()));
         // h_l = relu(conv(a_l; W1) + b1)
-        CTBB_TRY(conv_wgrad(c, d, c->a(l), c->du(), c->d_g + c->off_w[2 * l]));
-        bias_grad_kernel<<<grid1(ctx, n / 8 + 1), 256, 0, st>>>(n, c->du(), c->d_g + c->off_b[2 * l]);
-        CTBB_CUDA(cudaGetLastError());
+        CTBB_TRY(conv_wgrad(c, d, c->a(l), c->du(), c->d_g + c->off_w[2 * l], c->d_g + c->off_b[2 * l]));
         CTBB_TRY(conv_mid(c, d, c->du(), c->d_wb + (uint64_t)(2 * l) * kConvW, nullptr, g, nullptr, 0,
                           c->gbuf(1 - gi)));
         gi = 1 - gi;
     }
     // a_0 = relu(conv_in(s_in x) + b_in)
-    wgrad_1ch_kernel<<<wg_blocks, kWg1Threads, 0, st>>>(1, nx, ny, nz, c->gbuf(gi), x_dev, c->s_in, c->a(0),
-                                                         c->d_g + c->off_win);
+    wgrad_1ch_kernel<1><<<wg_blocks, 256, 0, st>>>(nx, ny, nz, w1x, w1y, w1tiles, c->gbuf(gi), x_dev, c->s_in,
+                                                   c->a(0), c->d_wpart);
+    CTBB_CUDA(cudaGetLastError());
+    wgrad_1ch_sum_kernel<1><<<kTaps + 1, 256, 0, st>>>(wg_blocks, c->d_wpart, c->d_g + c->off_win);
     CTBB_CUDA(cudaGetLastError());
     CTBB_CUDA(cudaStreamSynchronize(st));
     CTBB_TRY(check_conv_flag(c));
