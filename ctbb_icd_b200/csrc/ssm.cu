@@ -39,11 +39,18 @@ struct ViewTab {
     double off0, off1, off2;  // FFS deflection (zero without FFS)
 };
 
+// The same in FP32 and the channel tables in FP32, for the candidate filter.
+struct ViewTabF {
+    float src0, src1, src2, ew0, ew1, eu0, eu1, off0, off1, off2;
+};
+
 struct SsmParams {
     int nx, ny, nch, nr, nvsm, ffs;
     double vx, vy, vz, cvx, cvy, cvz;
-    double cc, dgam;  // channel centre and angular pitch (candidate search only)
-    double sa, cr;    // axial detector spacing and centre row (candidate search only)
+    // Candidate search and FP32 filter only: channel centre and angular pitch,
+    // axial detector spacing and centre row, reciprocal voxel sizes, and the
+    // filter's margins in voxels (in-plane, height).
+    float cc, rdgam, sa, cr, fvx, fvy, ivx, ivy, ivz, fcvx, fcvy, fcvz, tol, tolz;
 };
 
 // One candidate ray evaluated with the reference's arithmetic. Returns true
@@ -68,129 +75,160 @@ __device__ __forceinline__ bool ray_weight(const SsmParams& P, const ViewTab& V,
     d0 = d0 / n;
     d1 = d1 / n;
     d2 = d2 / n;
-    const double aax = fabs(d0), aay = fabs(d1);
-    if (aax > aay) {
-        // x-major: the ray is sampled on the line x = x_ic (generate_system_matrix.cpp:127-155).
-        const double x = (ic - P.cvx) * P.vx;
-        const double y_hat = V.src1 + d1 / d0 * (x - V.src0);
-        const double j_hat = y_hat / P.vy + P.cvy;
-        const int jj = (int)floor(j_hat);
-        if (jj != jc && jj != jc - 1) return false;
-        if (!(jj >= 0 && jj <= P.ny - 2)) return false;
-        const double z_hat = V.src2 + d2 / d0 * (x - V.src0);
-        const double k_hat = z_hat / P.vz + P.cvz;
-        const int kk = (int)floor(k_hat);
-        if (kk != -1 && kk != 0) return false;
-        const double scale = P.vx / aax;
-        const double wz = (kk == -1) ? scale * (k_hat - kk) : scale * (1 - (k_hat - kk));
-        *wout = (jj == jc) ? (float)(wz * (1 - (j_hat - jj))) : (float)(wz * (j_hat - jj));
-        return true;
-    } else {
-        // y-major: sampled on the line y = y_jc (generate_system_matrix.cpp:156-184).
-        const double y = (jc - P.cvy) * P.vy;
-        const double x_hat = V.src0 + d0 / d1 * (y - V.src1);
-        const double i_hat = x_hat / P.vx + P.cvx;
-        const int ii = (int)floor(i_hat);
-        if (ii != ic && ii != ic - 1) return false;
-        if (!(ii >= 0 && ii <= P.nx - 2)) return false;
-        const double z_hat = V.src2 + d2 / d1 * (y - V.src1);
-        const double k_hat = z_hat / P.vz + P.cvz;
-        const int kk = (int)floor(k_hat);
-        if (kk != -1 && kk != 0) return false;
-        const double scale = P.vy / aay;
-        const double wz = (kk == -1) ? scale * (k_hat - kk) : scale * (1 - (k_hat - kk));
-        *wout = (ii == ic) ? (float)(wz * (1 - (i_hat - ii))) : (float)(wz * (i_hat - ii));
-        return true;
-    }
+    // x-major rays are sampled on the line x = x_ic (generate_system_matrix.cpp:
+    // 127-155), y-major rays on y = y_jc (:156-184): the same expressions with
+    // the axes exchanged, evaluated once with the major axis selected so that
+    // the two quotients of each step run side by side (nearly every ray that
+    // gets here contributes, so there is nothing to gain from leaving early).
+    const bool xm = fabs(d0) > fabs(d1);
+    const double dm = xm ? d0 : d1, dn = xm ? d1 : d0;
+    const double line = xm ? (ic - P.cvx) * P.vx - V.src0 : (jc - P.cvy) * P.vy - V.src1;
+    const double n_hat = (xm ? V.src1 : V.src0) + dn / dm * line;
+    const double z_hat = V.src2 + d2 / dm * line;
+    const double j_hat = n_hat / (xm ? P.vy : P.vx) + (xm ? P.cvy : P.cvx);
+    const double k_hat = z_hat / P.vz + P.cvz;
+    const double scale = (xm ? P.vx : P.vy) / fabs(dm);
+    const int jj = (int)floor(j_hat), kk = (int)floor(k_hat);
+    const int own = xm ? jc : ic, last = (xm ? P.ny : P.nx) - 2;
+    const double wz = (kk == -1) ? scale * (k_hat - kk) : scale * (1 - (k_hat - kk));
+    *wout = (jj == own) ? (float)(wz * (1 - (j_hat - jj))) : (float)(wz * (j_hat - jj));
+    return (jj == own || jj == own - 1) && jj >= 0 && jj <= last && (kk == -1 || kk == 0);
 }
 
-// Approximate (fractional) channel whose ray passes through slice-frame point (px, py).
-__device__ __forceinline__ double chan_of(const SsmParams& P, const ViewTab& V, double px, double py) {
-    const double rx = px - V.src0, ry = py - V.src1;
-    const double a = -(rx * V.ew0 + ry * V.ew1);
-    const double b = -(rx * V.eu0 + ry * V.eu1);
-    return atan2(b, a) / P.dgam + P.cc;
+// Approximate (fractional) channel whose ray passes through slice-frame point
+// (px, py). FP32: off by under 1e-6 rad, a few thousandths of any real channel
+// pitch, where the candidate range is padded by a whole channel.
+__device__ __forceinline__ float chan_of(const SsmParams& P, const ViewTabF& V, float px, float py) {
+    const float rx = px - V.src0, ry = py - V.src1;
+    const float a = -(rx * V.ew0 + ry * V.ew1);
+    const float b = -(rx * V.eu0 + ry * V.eu1);
+    return atan2f(b, a) * P.rdgam + P.cc;
 }
 
-// Candidate rows for a ray with unnormalised in-plane component D (along
-// the sampling axis) reaching the sampling line at coordinate s from source
-// coordinate s0: z(k) = src2 - (k - cr) * sa * L with L = (s - s0) / D.
-__device__ __forceinline__ void row_range(const SsmParams& P, const ViewTab& V, double D, double s,
-                                          double s0, int* r_lo, int* r_hi) {
-    const double L = (s - s0) / D;
-    if (!(fabs(L) > 1e-12)) {
-        *r_lo = 0;
-        *r_hi = P.nr - 1;
-        return;
+// What FP32 arithmetic says of one channel's rays and column (ic, jc): rows
+// outside [r_lo, r_hi] do not contribute, rows in [s_lo, s_hi] do; the others lie
+// within the FP32 error of a boundary.
+struct Chan {
+    int r_lo, r_hi, s_lo, s_hi;
+};
+
+// Filter of one channel. The in-plane coordinate at which a ray crosses the
+// column's sampling line does not depend on the row (the direction's
+// normalisation cancels), so one FP32 evaluation per channel rejects a channel
+// whose rays pass outside [lo, hi) by more than `tol` voxels, and the ray's
+// height is linear in the row. Rays within 1e-4 of 45 degrees take the exact
+// test for every row (the major axis may differ per row).
+__device__ __forceinline__ Chan chan_filter(const SsmParams& P, const ViewTabF& V, float A, float B, float xc,
+                                            float yc, int ic, int jc) {
+    Chan c = {0, -1, 0, -1};
+    const float D0 = (A * V.ew0 - B * V.eu0) - V.off0;
+    const float D1 = (A * V.ew1 - B * V.eu1) - V.off1;
+    const float a0 = fabsf(D0), a1 = fabsf(D1);
+    const bool xm = a0 > a1;
+    // Major axis x: the ray crosses x = xc at parameter t (cm per unit of D), at
+    // u voxels along y, and contributes for u in [lo, hi). y: axes exchanged.
+    const float t = (xm ? xc - V.src0 : yc - V.src1) / (xm ? D0 : D1);
+    if (fabsf(a0 - a1) <= 1e-4f * fmaxf(a0, a1) || !(fabsf(t) > 1e-6f)) {
+        c.r_hi = P.nr - 1;
+        return c;
     }
-    // z(k) = src2 - ((k - cr) sa + off2) L: the z deflection of a z flying
-    // focal spot shifts the rows by -off2 / sa.
-    double a = V.src2 - P.vz, b = V.src2 + P.vz;  // k_hat in [-1, 1)  <=>  z in [-vz, vz)
-    double k0 = P.cr + a / (P.sa * L) - V.off2 / P.sa, k1 = P.cr + b / (P.sa * L) - V.off2 / P.sa;
-    if (k0 > k1) {
-        const double t = k0;
-        k0 = k1;
-        k1 = t;
+    const float u = ((xm ? V.src1 : V.src0) + (xm ? D1 : D0) * t) * (xm ? P.ivy : P.ivx) + (xm ? P.fcvy : P.fcvx);
+    const int own = xm ? jc : ic;
+    const float lo = (float)max(own - 1, 0), hi = (float)min(own + 1, (xm ? P.ny : P.nx) - 1);
+    if (u < lo - P.tol || u > hi + P.tol) return c;
+    // Height in voxels of row r's ray: (src2 - ((r - cr) sa + off2) t) / vz + cvz
+    // (the z deflection of a z flying focal spot shifts it by off2 t); heights in
+    // [-1, 1) contribute.
+    const float sz = t * P.ivz;
+    const float z0 = (V.src2 * P.ivz + P.fcvz) + (P.cr * P.sa - V.off2) * sz;
+    const float rdz = -1.f / (P.sa * sz);
+    const float k0 = (-1.f - z0) * rdz, k1 = (1.f - z0) * rdz;
+    const float ka = fminf(k0, k1), kb = fmaxf(k0, k1), d = P.tolz * fabsf(rdz) + 1e-3f;
+    const float last = (float)(P.nr - 1);
+    c.r_lo = (int)fmaxf(ceilf(ka - d), 0.f);
+    c.r_hi = (int)fminf(floorf(kb + d), last);
+    if (u > lo + P.tol && u < hi - P.tol) {
+        c.s_lo = (int)fmaxf(ceilf(ka + d), 0.f);
+        c.s_hi = (int)fminf(floorf(kb - d), last);
     }
-    int lo = (int)floor(k0) - 1, hi = (int)ceil(k1) + 1;
-    *r_lo = max(lo, 0);
-    *r_hi = min(hi, P.nr - 1);
+    return c;
 }
 
+// One thread per (column, view) cell. What bounds it: FP64 divisions. An exact
+// evaluation of one ray costs a square root and eight of them, and the padded
+// candidate ranges hold some 50 rays per cell of which 2 or 3 contribute, so the
+// FP32 filter above decides every ray that is clearly in or out: the fill
+// evaluates only the rays that contribute (it needs their weights) and the few
+// within the FP32 error of a boundary, the count only the latter.
 template <bool FILL>
 __global__ void __launch_bounds__(256) ssm_cells_kernel(
-    SsmParams P, const ViewTab* __restrict__ vt, const double* __restrict__ chA,
-    const double* __restrict__ chB, const double* __restrict__ rowAp, const double* __restrict__ rowN,
-    uint16_t* __restrict__ cnt, const int64_t* __restrict__ colptr, const uint32_t* __restrict__ vptr,
-    int32_t* __restrict__ idx, float* __restrict__ w32, __half* __restrict__ w16) {
-    const uint64_t ncell = (uint64_t)P.nx * P.ny * P.nvsm;
-    for (uint64_t cell = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; cell < ncell;
-         cell += (uint64_t)gridDim.x * blockDim.x) {
-        const int v = (int)(cell % P.nvsm);
-        const uint64_t col = cell / P.nvsm;
+    SsmParams P, const ViewTab* __restrict__ vt, const ViewTabF* __restrict__ vtf, const double* __restrict__ chA,
+    const double* __restrict__ chB, const float2* __restrict__ chF, const double* __restrict__ rowAp,
+    const double* __restrict__ rowN, uint16_t* __restrict__ cnt, const int64_t* __restrict__ colptr,
+    const uint32_t* __restrict__ vptr, int32_t* __restrict__ idx, float* __restrict__ w32,
+    __half* __restrict__ w16) {
+    // A block walks a column's views: no divisions per cell, and neighbouring
+    // lanes meet neighbouring channels and rows.
+    const uint64_t ncol = (uint64_t)P.nx * P.ny;
+    const int vblocks = (P.nvsm + 255) / 256;
+    for (uint64_t unit = blockIdx.x; unit < ncol * vblocks; unit += gridDim.x) {
+        const uint64_t col = unit / (uint32_t)vblocks;
+        const int v = (int)(unit - col * vblocks) * 256 + (int)threadIdx.x;
+        if (v >= P.nvsm) continue;
+        const uint64_t cell = col * P.nvsm + v;
         const int ic = (int)(col % P.nx), jc = (int)(col / P.nx);
-        const ViewTab V = vt[v];
+        const ViewTabF V = vtf[v];
         // Candidate channels: rays through the two sampling segments of this
         // column (vertical at x_ic for x-major rays, horizontal at y_jc for
         // y-major rays), padded by one channel for rounding and by three with
         // a flying focal spot (the deflected source shifts a ray by about a
         // channel at the fan edge relative to the nominal fan model used for
         // the bound).
-        const double xc = (ic - P.cvx) * P.vx, yc = (jc - P.cvy) * P.vy;
-        const double c0 = chan_of(P, V, xc, yc - P.vy), c1 = chan_of(P, V, xc, yc + P.vy);
-        const double c2 = chan_of(P, V, xc - P.vx, yc), c3 = chan_of(P, V, xc + P.vx, yc);
-        const double cmin = fmin(fmin(c0, c1), fmin(c2, c3)), cmax = fmax(fmax(c0, c1), fmax(c2, c3));
+        const float xc = (float)((ic - P.cvx) * P.vx), yc = (float)((jc - P.cvy) * P.vy);
+        const float c0 = chan_of(P, V, xc, yc - P.fvy), c1 = chan_of(P, V, xc, yc + P.fvy);
+        const float c2 = chan_of(P, V, xc - P.fvx, yc), c3 = chan_of(P, V, xc + P.fvx, yc);
+        const float cmin = fminf(fminf(c0, c1), fminf(c2, c3)), cmax = fmaxf(fmaxf(c0, c1), fmaxf(c2, c3));
         const int pad = P.ffs ? 3 : 1;
-        const int ch_lo = max((int)floor(cmin) - pad, 0);
-        const int ch_hi = min((int)ceil(cmax) + pad, P.nch - 1);
+        const int ch_lo = max((int)floorf(cmin) - pad, 0);
+        const int ch_hi = min((int)ceilf(cmax) + pad, P.nch - 1);
         uint32_t n = 0;
         int64_t base = 0;
         if (FILL) base = colptr[col] + (int64_t)vptr[col * (uint64_t)(P.nvsm + 1) + v];
         const int q_view = P.nr * P.nch * v;
-        for (int ch = ch_lo; ch <= ch_hi; ++ch) {
-            const double A = chA[ch], B = chB[ch];
-            const double D0 = (A * V.ew0 - B * V.eu0) - V.off0;
-            const double D1 = (A * V.ew1 - B * V.eu1) - V.off1;
-            int r_lo, r_hi;
-            const double ad0 = fabs(D0), ad1 = fabs(D1);
-            if (fabs(ad0 - ad1) <= 1e-9 * fmax(ad0, ad1)) {
-                r_lo = 0;  // near 45 degrees: the major axis may differ per row
-                r_hi = P.nr - 1;
-            } else if (ad0 > ad1) {
-                row_range(P, V, D0, xc, V.src0, &r_lo, &r_hi);
-            } else {
-                row_range(P, V, D1, yc, V.src1, &r_lo, &r_hi);
-            }
-            for (int r = r_lo; r <= r_hi; ++r) {
-                float w;
-                if (ray_weight(P, V, A, B, rowAp[r], rowN[r], ic, jc, &w)) {
-                    if (FILL) {
-                        const int64_t o = base + n;
-                        idx[o] = r + P.nr * ch + q_view;
-                        if (w32) w32[o] = w;
-                        if (w16) w16[o] = __float2half_rn(w);
-                    }
+        float w;
+        if (FILL) {
+            int ch = ch_lo - 1, r = 0, r_hi = -1;
+            for (;;) {
+                // Advance to the next ray, then evaluate it: a warp's lanes meet
+                // their n-th rays together.
+                while (r > r_hi) {
+                    if (++ch > ch_hi) break;
+                    const float2 ab = chF[ch];
+                    const Chan c = chan_filter(P, V, ab.x, ab.y, xc, yc, ic, jc);
+                    r = c.r_lo;
+                    r_hi = c.r_hi;
+                }
+                if (ch > ch_hi) break;
+                if (ray_weight(P, vt[v], chA[ch], chB[ch], rowAp[r], rowN[r], ic, jc, &w)) {
+                    const int64_t o = base + n;
+                    idx[o] = r + P.nr * ch + q_view;
+                    if (w32) w32[o] = w;
+                    if (w16) w16[o] = __float2half_rn(w);
                     ++n;
+                }
+                ++r;
+            }
+        } else {
+            for (int ch = ch_lo; ch <= ch_hi; ++ch) {
+                const float2 ab = chF[ch];
+                const Chan c = chan_filter(P, V, ab.x, ab.y, xc, yc, ic, jc);
+                n += (uint32_t)max(c.s_hi - c.s_lo + 1, 0);
+                for (int r = c.r_lo; r <= c.r_hi; ++r) {
+                    if (r >= c.s_lo && r <= c.s_hi) {
+                        r = c.s_hi;
+                        continue;
+                    }
+                    n += ray_weight(P, vt[v], chA[ch], chB[ch], rowAp[r], rowN[r], ic, jc, &w) ? 1u : 0u;
                 }
             }
         }
@@ -540,10 +578,29 @@ extern "C" ctbb_status ctbb_gpu_generate_ssm(ctbb_ctx* ctx, const ctbb_geom_c* g
     P.cvx = g.center_voxel_x;
     P.cvy = g.center_voxel_y;
     P.cvz = g.center_voxel_z;
-    P.cc = g.center_channel_non_ffs;
-    P.dgam = ffs ? g.fan_angle_increment : g.transaxial_detector_spacing / g.source_detector_distance;
-    P.sa = g.axial_detector_spacing;
-    P.cr = g.center_row;
+    P.cc = (float)g.center_channel_non_ffs;
+    P.rdgam = (float)(1.0 / (ffs ? g.fan_angle_increment : g.transaxial_detector_spacing / g.source_detector_distance));
+    P.fvx = (float)g.voxel_size_x;
+    P.fvy = (float)g.voxel_size_y;
+    P.fcvx = (float)g.center_voxel_x;
+    P.fcvy = (float)g.center_voxel_y;
+    P.fcvz = (float)g.center_voxel_z;
+    P.sa = (float)g.axial_detector_spacing;
+    P.cr = (float)g.center_row;
+    P.ivx = (float)(1.0 / g.voxel_size_x);
+    P.ivy = (float)(1.0 / g.voxel_size_y);
+    P.ivz = (float)(1.0 / g.voxel_size_z);
+    // FP32 positions are off by up to four roundings of the lengths they are
+    // made of: the source radius and the field of view in-plane, those times the
+    // rays' slope and the source's travel in z. The margins are four times that
+    // and a thousandth of a voxel.
+    double zmax = 0.0;
+    for (const ViewTab& t : hv) zmax = std::max(zmax, fabs(t.src2));
+    const double reach = 2.0 * (g.focal_spot_radius + g.voxel_size_x * P.nx + g.voxel_size_y * P.ny);
+    const double slope = 2.0 * (fabs(g.center_row) + (double)P.nr) * g.axial_detector_spacing / g.source_detector_distance;
+    const double ulp = 16.0 / 16777216.0;
+    P.tol = (float)(1e-3 + ulp * (reach / std::min(g.voxel_size_x, g.voxel_size_y) + P.nx + P.ny));
+    P.tolz = (float)(1e-3 + ulp * (zmax + reach * slope) / g.voxel_size_z);
 
     Scoped tmp;
     ViewTab* d_vt = nullptr;
@@ -554,6 +611,20 @@ extern "C" ctbb_status ctbb_gpu_generate_ssm(ctbb_ctx* ctx, const ctbb_geom_c* g
     tmp.ptrs.push_back(d_A);
     CTBB_TRY(upload(hB, &d_B, st));
     tmp.ptrs.push_back(d_B);
+    std::vector<ViewTabF> hvf(hv.size());
+    for (size_t i = 0; i < hv.size(); ++i) {
+        const ViewTab& t = hv[i];
+        hvf[i] = {(float)t.src0, (float)t.src1, (float)t.src2, (float)t.ew0, (float)t.ew1,
+                  (float)t.eu0,  (float)t.eu1,  (float)t.off0, (float)t.off1, (float)t.off2};
+    }
+    std::vector<float2> hF(hA.size());
+    for (size_t i = 0; i < hF.size(); ++i) hF[i] = make_float2((float)hA[i], (float)hB[i]);
+    ViewTabF* d_vtf = nullptr;
+    float2* d_F = nullptr;
+    CTBB_TRY(upload(hvf, &d_vtf, st));
+    tmp.ptrs.push_back(d_vtf);
+    CTBB_TRY(upload(hF, &d_F, st));
+    tmp.ptrs.push_back(d_F);
     CTBB_TRY(upload(hap, &d_ap, st));
     tmp.ptrs.push_back(d_ap);
     CTBB_TRY(upload(hn, &d_n, st));
@@ -592,7 +663,7 @@ extern "C" ctbb_status ctbb_gpu_generate_ssm(ctbb_ctx* ctx, const ctbb_geom_c* g
     CTBB_CUDA(cudaEventCreate(&e1));
     CTBB_CUDA(cudaEventRecord(e0, st));
     const int grid = grid_for(ctx, ncell, 256);
-    ssm_cells_kernel<false><<<grid, 256, 0, st>>>(P, d_vt, d_A, d_B, d_ap, d_n, d_cnt, nullptr, nullptr,
+    ssm_cells_kernel<false><<<grid, 256, 0, st>>>(P, d_vt, d_vtf, d_A, d_B, d_F, d_ap, d_n, d_cnt, nullptr, nullptr,
                                                   nullptr, nullptr, nullptr);
     CTBB_CUDA(cudaGetLastError());
     ssm_column_scan_kernel<<<(int)std::min<uint64_t>(s->ncol, (uint64_t)ctx->sm_count * 32), 256, 0, st>>>(
@@ -611,7 +682,7 @@ extern "C" ctbb_status ctbb_gpu_generate_ssm(ctbb_ctx* ctx, const ctbb_geom_c* g
     CTBB_CUDA(cudaMalloc(&s->d_idx, nalloc * sizeof(int32_t)));
     if (weights & CTBB_SSM_FP32) CTBB_CUDA(cudaMalloc(&s->d_w32, nalloc * sizeof(float)));
     if (weights & CTBB_SSM_FP16) CTBB_CUDA(cudaMalloc(&s->d_w16, nalloc * sizeof(__half)));
-    ssm_cells_kernel<true><<<grid, 256, 0, st>>>(P, d_vt, d_A, d_B, d_ap, d_n, nullptr, s->d_colptr,
+    ssm_cells_kernel<true><<<grid, 256, 0, st>>>(P, d_vt, d_vtf, d_A, d_B, d_F, d_ap, d_n, nullptr, s->d_colptr,
                                                  s->d_vptr, s->d_idx, s->d_w32, s->d_w16);
     CTBB_CUDA(cudaGetLastError());
     CTBB_CUDA(cudaEventRecord(e1, st));
