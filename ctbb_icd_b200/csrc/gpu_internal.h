@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 #include <vector>
 
@@ -45,8 +46,69 @@ struct ctbb_ctx {
     int* d_flags = nullptr;  // device-side error flags
 };
 
+// Layout of sinograms on the device (error sinogram, FP64 estimate) and of the
+// matrix's sinogram indices: views fastest but for groups of 2^rb detector rows,
+//   ((channel * nrb + (row >> rb)) * stride + view) << rb | row low bits.
+// What bounds the kernels that read it is not bytes but requests: a voxel meets
+// one or two channels and two rows per view, and its channel drifts slowly from
+// view to view, so in the raw data's order (row fastest) neighbouring entries each
+// lie in another 128-byte line. Here a line holds 8 views of 4 rows: the 16 entry
+// pairs of a warp's load touch 6.3 lines instead of 15.5 and 13.7 sectors instead
+// of 17 (512 x 512 x 64 benchmark; 9.6 and 14 on 2.3 mm voxels). A slice's first
+// view still adds a constant (s << rb) to every index of a column, which a blocked
+// order with view blocks does not give. Rows are padded to whole groups, views to
+// whole lines; padding holds zeros. Where that would not fit a 31-bit index, rb
+// is 0 and nothing is padded.
+struct SinoLayout {
+    int rb = 0, nr = 0, nch = 0, nrb = 0;
+    uint32_t stride = 0;  // views, padded
+
+    static SinoLayout make(uint64_t nch, uint64_t nr, uint64_t views) {
+        SinoLayout l;
+        l.nr = (int)nr;
+        l.nch = (int)nch;
+        l.rb = nr >= 3 ? 2 : (int)nr - 1;
+        l.nrb = (l.nr + (1 << l.rb) - 1) >> l.rb;
+        l.stride = (uint32_t)((views + 7) / 8 * 8);
+        if (l.size() >= 2147483648ull) {
+            l.rb = 0;
+            l.nrb = l.nr;
+            l.stride = (uint32_t)views;
+        }
+        return l;
+    }
+    uint64_t size() const { return ((uint64_t)nch * nrb * stride) << rb; }
+    __host__ __device__ uint32_t at(uint32_t view, uint32_t ch, uint32_t row) const {
+        return (((ch * (uint32_t)nrb + (row >> rb)) * stride + view) << rb) | (row & ((1u << rb) - 1u));
+    }
+    // The inverse; rows and views of the padding come out past the end.
+    __host__ __device__ void split(uint32_t a, uint32_t* view, uint32_t* ch, uint32_t* row) const {
+        const uint32_t t = a >> rb, u = t / stride, c = u / (uint32_t)nrb;
+        *view = t - u * stride;
+        *ch = c;
+        *row = ((u - c * (uint32_t)nrb) << rb) | (a & ((1u << rb) - 1u));
+    }
+    // The raw data's order (row fastest).
+    __host__ __device__ uint32_t linear(uint32_t a) const {
+        uint32_t v, c, r;
+        split(a, &v, &c, &r);
+        return r + (uint32_t)nr * (c + (uint32_t)nch * v);
+    }
+    __host__ __device__ uint32_t from_linear(uint32_t q) const {
+        const uint32_t t = q / (uint32_t)nr, v = t / (uint32_t)nch;
+        return at(v, t - v * (uint32_t)nch, q - t * (uint32_t)nr);
+    }
+    // What leads from a row to the next one of the same view and channel: 1 within
+    // a group, row_step() from its last row (low bits all ones) to the next group.
+    __host__ __device__ uint32_t row_mask() const { return (1u << rb) - 1u; }
+    __host__ __device__ uint32_t row_step() const { return (stride << rb) - row_mask(); }
+    bool operator==(const SinoLayout& o) const {
+        return rb == o.rb && nr == o.nr && nch == o.nch && stride == o.stride;
+    }
+};
+
 // Stored system matrix: per voxel column c = i + nx*j, entries sorted by
-// q = row + Nrows*(channel + n_channels*view). colptr[c] is the first entry of
+// q = row + Nrows*(channel + n_channels*view), stored as lay.from_linear(q). colptr[c] is the first entry of
 // column c; vptr[c*(nvsm+1) + v] is the offset (relative to colptr[c]) of the
 // first entry of SSM view v, so a view window [v0, v1) is one contiguous run.
 struct ctbb_ssm {
@@ -60,6 +122,7 @@ struct ctbb_ssm {
         return ++n;
     }
     ctbb_geom_c geom{};
+    SinoLayout lay;
     uint64_t ncol = 0, nvsm = 0, nnz = 0, max_col_nnz = 0;
     int64_t* d_colptr = nullptr;  // [ncol + 1]
     uint32_t* d_vptr = nullptr;   // [ncol * (nvsm + 1)]
@@ -72,7 +135,7 @@ struct ctbb_ssm {
     int64_t* d_pcolptr = nullptr;  // [ncol + 1]
     uint32_t* d_pvptr = nullptr;   // [ncol * (nvsm + 1)]
     uint2* d_pairs = nullptr;      // [npairs]
-    uint64_t npairs = 0;
+    uint64_t npairs = 0;       // runs of two consecutive q (reported)
     bool pairs_checked = false;  // build tried (pairs kept only where they pay)
     int weights = 0;
     int ffs = 0;
@@ -86,14 +149,16 @@ struct ctbb_ssm {
 struct ctbb_recon {
     ctbb_ctx* ctx = nullptr;
     ctbb_geom_c geom{};
+    SinoLayout lay;
     uint64_t nvox = 0, data_size = 0;
+    uint64_t sino_size = 0;  // elements of d_est64 and d_e32 (lay.size())
     std::vector<uint64_t> slice_indices;
     int32_t* d_start = nullptr;  // [nz] first data view of each slice's SSM window
     float* d_raw = nullptr;      // y
     double* d_x64 = nullptr;     // sequential-mode image
     double* d_est64 = nullptr;   // sequential-mode A x (FP64); also FP64 refresh accumulator
     float* d_x32 = nullptr;      // grouped-mode image
-    float* d_e32 = nullptr;      // grouped-mode y - A x
+    float* d_e32 = nullptr;      // grouped-mode y - A x; sequential mode: y in the same layout
     int rep = 0;                 // 0: x64/est64 current, 1: x32/e32 current
     // Sum over voxels inside the FOV of in-range matrix entries (cached per matrix).
     uint64_t entries_ssm = 0;
@@ -133,10 +198,13 @@ ctbb_status ensure_partials(ctbb_ctx* ctx, size_t n);
 // ssm.cu
 ctbb_status ssm_validate_geometry(const ctbb_geom_c& g);
 ctbb_status ssm_build_pairs(ctbb_ssm* s);
+ctbb_status ssm_relayout(ctbb_ssm* s, const SinoLayout& to);
 
 // recon.cu
 ctbb_status recon_to_grouped(ctbb_recon* rc, const ctbb_ssm* ssm);
 ctbb_status recon_to_sequential(ctbb_recon* rc, const ctbb_ssm* ssm);
+ctbb_status arranged_raw(ctbb_recon* rc);  // y in the device layout into d_e32
+ctbb_status match_layout(ctbb_recon* rc, const ctbb_ssm* ssm);
 ctbb_status forward_project_f64(ctbb_recon* rc, const ctbb_ssm* ssm, bool from_x32, double* d_out);
 ctbb_status cost_f64(ctbb_recon* rc, const ctbb_ssm* ssm, bool exact, double* out);
 

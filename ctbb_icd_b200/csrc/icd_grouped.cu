@@ -60,7 +60,9 @@
 namespace {
 
 struct GParams {
-    int nx, ny, nz, nch, nr, nvsm, readings, penalty;
+    int nx, ny, nz, nvsm, readings, penalty;
+    int rb;                    // sinogram layout: a slice's first view adds s << rb to its indices,
+    uint32_t row_mask, row_step;  // and the next detector row is 1 or row_step further (SinoLayout)
     int last_slice[2];  // last slice of each parity
     uint64_t n_items, nvsm1;
     double lambda, delta;
@@ -145,6 +147,12 @@ __device__ __forceinline__ void load_chunk(const int32_t* __restrict__ idx, cons
             wt[u] = 0.f;
         }
     }
+}
+
+// Sinogram index of a pair's entry: the pair's own row a, or the next one.
+__device__ __forceinline__ int pair_index(const GParams& P, uint32_t a, int off, int half) {
+    const uint32_t step = (a & P.row_mask) == P.row_mask ? P.row_step : 1u;
+    return (int)a + off + (half ? (int)step : 0);
 }
 
 // The two FP16 weights of an entry pair ({q, w0 | w1 << 16}).
@@ -452,7 +460,7 @@ __device__ __forceinline__ void process_item(const GParams& P, const uint32_t* _
         const int vs = min(max(start[kl] - s, v0), v1);
         mid = cb + vp[vs];
     }
-    const int off = s * P.nch * P.nr;
+    const int off = s * (1 << P.rb);
 
     // beta = sum a e, alpha = sum a^2 (FP32 accumulation per lane) over
     // [mid, en) then [b, mid).
@@ -517,7 +525,7 @@ __global__ void __launch_bounds__(256) icd_grouped_kernel(GParams P, const uint3
 // matrix costs 4 bytes per entry instead of 6. Position p of a lane in row u
 // of a chunk: pair base + 16 u + lane / 2, entry lane & 1.
 template <int U, int STRIDE = 16>
-__device__ __forceinline__ void load_pair_entries(const uint2* __restrict__ pairs, int64_t m, int64_t en, int off,
+__device__ __forceinline__ void load_pair_entries(const GParams& P, const uint2* __restrict__ pairs, int64_t m, int64_t en, int off,
                                                   int half, uint64_t pol, int* q, float* wt) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -530,7 +538,7 @@ __device__ __forceinline__ void load_pair_entries(const uint2* __restrict__ pair
                          : "=r"(a), "=r"(bb)
                          : "l"(pairs + mu), "l"(pol));
             if (!half || (bb >> 16)) {
-                q[u] = (int)a + off + half;
+                q[u] = pair_index(P, a, off, half);
                 wt[u] = half ? half_hi(bb) : half_lo(bb);
             }
         }
@@ -540,7 +548,7 @@ __device__ __forceinline__ void load_pair_entries(const uint2* __restrict__ pair
 // Pair positions p, p + STRIDE, ... of an item's sweep: pair p + hi for
 // p < n1, else p + lo; -1 / 0 past n (the sweep's length).
 template <int U, int STRIDE>
-__device__ __forceinline__ void load_seq_pairs(const uint2* __restrict__ pairs, int p0, int n, int n1, int64_t hi,
+__device__ __forceinline__ void load_seq_pairs(const GParams& P, const uint2* __restrict__ pairs, int p0, int n, int n1, int64_t hi,
                                                int64_t lo, int off, int half, uint64_t pol, int* q, float* wt) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -554,7 +562,7 @@ __device__ __forceinline__ void load_seq_pairs(const uint2* __restrict__ pairs, 
                          : "=r"(a), "=r"(bb)
                          : "l"(pairs + m), "l"(pol));
             if (!half || (bb >> 16)) {
-                q[u] = (int)a + off + half;
+                q[u] = pair_index(P, a, off, half);
                 wt[u] = half ? half_hi(bb) : half_lo(bb);
             }
         }
@@ -562,20 +570,20 @@ __device__ __forceinline__ void load_seq_pairs(const uint2* __restrict__ pairs, 
 }
 
 template <int U>
-__device__ __forceinline__ void gather_pairs(const uint2* __restrict__ pairs, const float* e, int64_t b, int64_t en,
+__device__ __forceinline__ void gather_pairs(const GParams& P, const uint2* __restrict__ pairs, const float* e, int64_t b, int64_t en,
                                              int off, int lane, uint64_t pol, float& acc_b, float& acc_a) {
     if (b >= en) return;
     const int half = lane & 1, j = lane >> 1;
     int qa[U];
     float wa[U];
-    load_pair_entries<U>(pairs, b + j, en, off, half, pol, qa, wa);
+    load_pair_entries<U>(P, pairs, b + j, en, off, half, pol, qa, wa);
     for (int64_t base = b; base < en; base += 16 * U) {
         float ev[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) ev[u] = qa[u] >= 0 ? __ldcg(e + qa[u]) : 0.f;
         int qb[U];
         float wb[U];
-        load_pair_entries<U>(pairs, base + 16 * U + j, en, off, half, pol, qb, wb);
+        load_pair_entries<U>(P, pairs, base + 16 * U + j, en, off, half, pol, qb, wb);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             acc_b = fmaf(wa[u], ev[u], acc_b);
@@ -587,7 +595,7 @@ __device__ __forceinline__ void gather_pairs(const uint2* __restrict__ pairs, co
 }
 
 template <int U>
-__device__ __forceinline__ void scatter_pairs(const uint2* __restrict__ pairs, float* e, int64_t b, int64_t en,
+__device__ __forceinline__ void scatter_pairs(const GParams& P, const uint2* __restrict__ pairs, float* e, int64_t b, int64_t en,
                                               int off, int lane, uint64_t pol, float du) {
     if (b >= en) return;
     const int half = lane & 1, j = lane >> 1;
@@ -595,7 +603,7 @@ __device__ __forceinline__ void scatter_pairs(const uint2* __restrict__ pairs, f
     for (int64_t c = nchunk - 1; c >= 0; --c) {
         int qs[U];
         float ws[U];
-        load_pair_entries<U>(pairs, b + c * (16 * U) + j, en, off, half, pol, qs, ws);
+        load_pair_entries<U>(P, pairs, b + c * (16 * U) + j, en, off, half, pol, qs, ws);
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (qs[u] >= 0) atomicAdd(e + qs[u], -du * ws[u]);
@@ -634,11 +642,11 @@ __global__ void __launch_bounds__(256) icd_grouped_pairs_kernel(
             mid = cb + vp[min(max(start[kl] - s, v0), v1)];
             n_entries = (int64_t)vptr[col * P.nvsm1 + v1] - (int64_t)vptr[col * P.nvsm1 + v0];
         }
-        const int off = s * P.nch * P.nr;
+        const int off = s * (1 << P.rb);
         float acc_b = 0.f, acc_a = 0.f;
         const uint64_t keep = l2_keep();
-        gather_pairs<U>(pairs, e, mid, en, off, lane, keep, acc_b, acc_a);
-        gather_pairs<U>(pairs, e, b, mid, off, lane, keep, acc_b, acc_a);
+        gather_pairs<U>(P, pairs, e, mid, en, off, lane, keep, acc_b, acc_a);
+        gather_pairs<U>(P, pairs, e, b, mid, off, lane, keep, acc_b, acc_a);
         const double beta = (double)warp_sum(acc_b);
         const double alpha = (double)warp_sum(acc_a);
         const double xq = (double)__ldcg(x + q);
@@ -648,8 +656,8 @@ __global__ void __launch_bounds__(256) icd_grouped_pairs_kernel(
         const float du = (float)upd;
         if (du != 0.f) {
             const uint64_t drop = l2_drop();
-            scatter_pairs<U>(pairs, e, b, mid, off, lane, drop, du);
-            scatter_pairs<U>(pairs, e, mid, en, off, lane, drop, du);
+            scatter_pairs<U>(P, pairs, e, b, mid, off, lane, drop, du);
+            scatter_pairs<U>(P, pairs, e, mid, en, off, lane, drop, du);
             n_ent += (unsigned long long)n_entries;
             ++n_upd;
         }
@@ -723,7 +731,7 @@ __global__ void __launch_bounds__(32 * WPV, 16 / WPV) icd_cta_pairs_kernel(
             mid = P.stack_align ? cb + vp[stack_start_view(P, start, k, s, v0, v1)] : b;
             if (tid == 0) n_entries = (int64_t)vptr[col * P.nvsm1 + v1] - (int64_t)vptr[col * P.nvsm1 + v0];
         }
-        const int off = s * P.nch * P.nr;
+        const int off = s * (1 << P.rb);
         // Sweep position p (pairs) -> pair p + hi for p < n1 ([mid, en)), else
         // p + lo ([b, mid)).
         const int n = (int)(en - b), n1 = (int)(en - mid);
@@ -743,7 +751,7 @@ __global__ void __launch_bounds__(32 * WPV, 16 / WPV) icd_cta_pairs_kernel(
                              : "=r"(a), "=r"(bb)
                              : "l"(pairs + m), "l"(pol_m));
                 if (!half || (bb >> 16)) {
-                    qr[r] = (int)a + off + half;
+                    qr[r] = pair_index(P, a, off, half);
                     wr[r] = half ? half_hi(bb) : half_lo(bb);
                 }
             }
@@ -758,7 +766,7 @@ __global__ void __launch_bounds__(32 * WPV, 16 / WPV) icd_cta_pairs_kernel(
         for (int base = (int)CAP; base < n; base += NP * kU) {
             int qo[kU];
             float wo[kU];
-            load_seq_pairs<kU, NP>(pairs, base + j, n, n1, hi, lo, off, half, pol_m, qo, wo);
+            load_seq_pairs<kU, NP>(P, pairs, base + j, n, n1, hi, lo, off, half, pol_m, qo, wo);
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
                 const float ev = qo[u] >= 0 ? ld_e(e + qo[u], pol_e) : 0.f;
@@ -797,7 +805,7 @@ __global__ void __launch_bounds__(32 * WPV, 16 / WPV) icd_cta_pairs_kernel(
             for (int base = (int)CAP; base < n; base += NP * kU) {
                 int qo[kU];
                 float wo[kU];
-                load_seq_pairs<kU, NP>(pairs, base + j, n, n1, hi, lo, off, half, pol_m, qo, wo);
+                load_seq_pairs<kU, NP>(P, pairs, base + j, n, n1, hi, lo, off, half, pol_m, qo, wo);
 #pragma unroll
                 for (int u = 0; u < kU; ++u)
                     if (qo[u] >= 0) atomicAdd(e + qo[u], -du * wo[u]);
@@ -914,7 +922,7 @@ __device__ __forceinline__ void bulk_issue(const GParams& P, const uint32_t* __r
     it->en = en;
     it->q = (int64_t)col + (int64_t)ncol * k;
     it->n_entries = ne;
-    it->off = s * P.nch * P.nr;
+    it->off = s * (1 << P.rb);
     it->d = (int)(b - b0);
     it->ns = ns;
     it->valid = 1;
@@ -987,7 +995,7 @@ __global__ void __launch_bounds__(kBulkThreads, STAGES == 1 ? 4 : 3) icd_bulk_ke
             float v = 0.f;
             if (p < it.ns) {
                 const uint2 pr = stp[p];
-                if (!half || (pr.y >> 16)) v = __ldcg(e + ((int)pr.x + it.off + half));
+                if (!half || (pr.y >> 16)) v = __ldcg(e + pair_index(P, pr.x, it.off, half));
             }
             ev[i] = v;
         }
@@ -1005,7 +1013,7 @@ __global__ void __launch_bounds__(kBulkThreads, STAGES == 1 ? 4 : 3) icd_bulk_ke
         for (int b2 = it.ns; b2 < n; b2 += kBulkNP * kU) {
             int qo[kU];
             float wo[kU];
-            load_pair_entries<kU, kBulkNP>(pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
+            load_pair_entries<kU, kBulkNP>(P, pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
                 const float evu = qo[u] >= 0 ? __ldcg(e + qo[u]) : 0.f;
@@ -1045,13 +1053,13 @@ __global__ void __launch_bounds__(kBulkThreads, STAGES == 1 ? 4 : 3) icd_bulk_ke
                 if (p < it.ns) {
                     const uint2 pr = stp[p];
                     if (!half || (pr.y >> 16))
-                        atomicAdd(e + ((int)pr.x + it.off + half), -du * (half ? half_hi(pr.y) : half_lo(pr.y)));
+                        atomicAdd(e + pair_index(P, pr.x, it.off, half), -du * (half ? half_hi(pr.y) : half_lo(pr.y)));
                 }
             }
             for (int b2 = it.ns; b2 < n; b2 += kBulkNP * kU) {
                 int qo[kU];
                 float wo[kU];
-                load_pair_entries<kU, kBulkNP>(pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
+                load_pair_entries<kU, kBulkNP>(P, pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
 #pragma unroll
                 for (int u = 0; u < kU; ++u)
                     if (qo[u] >= 0) atomicAdd(e + qo[u], -du * wo[u]);
@@ -1119,7 +1127,7 @@ __device__ __forceinline__ void bulk_claim(const GParams& P, const uint32_t* __r
     it->en = en;
     it->q = (int64_t)col + (int64_t)ncol * k;
     it->n_entries = ne;
-    it->off = s * P.nch * P.nr;
+    it->off = s * (1 << P.rb);
     it->d = (int)(b - (b & ~(int64_t)1));
     it->ns = ns;
     it->valid = 1;
@@ -1193,7 +1201,7 @@ __global__ void __launch_bounds__(kBulkThreads, 4) icd_bulk_pipe_kernel(
             float v = 0.f;
             if (p < it.ns) {
                 const uint2 pr = stp[p];
-                if (!half || (pr.y >> 16)) v = __ldcg(e + ((int)pr.x + it.off + half));
+                if (!half || (pr.y >> 16)) v = __ldcg(e + pair_index(P, pr.x, it.off, half));
             }
             ev[i] = v;
         }
@@ -1211,7 +1219,7 @@ __global__ void __launch_bounds__(kBulkThreads, 4) icd_bulk_pipe_kernel(
         for (int b2 = it.ns; b2 < n; b2 += kBulkNP * kU) {
             int qo[kU];
             float wo[kU];
-            load_pair_entries<kU, kBulkNP>(pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
+            load_pair_entries<kU, kBulkNP>(P, pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
                 const float evu = qo[u] >= 0 ? __ldcg(e + qo[u]) : 0.f;
@@ -1255,13 +1263,13 @@ __global__ void __launch_bounds__(kBulkThreads, 4) icd_bulk_pipe_kernel(
                 if (p < it.ns) {
                     const uint2 pr = stp[p];
                     if (!half || (pr.y >> 16))
-                        atomicAdd(e + ((int)pr.x + it.off + half), -du * (half ? half_hi(pr.y) : half_lo(pr.y)));
+                        atomicAdd(e + pair_index(P, pr.x, it.off, half), -du * (half ? half_hi(pr.y) : half_lo(pr.y)));
                 }
             }
             for (int b2 = it.ns; b2 < n; b2 += kBulkNP * kU) {
                 int qo[kU];
                 float wo[kU];
-                load_pair_entries<kU, kBulkNP>(pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
+                load_pair_entries<kU, kBulkNP>(P, pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
 #pragma unroll
                 for (int u = 0; u < kU; ++u)
                     if (qo[u] >= 0) atomicAdd(e + qo[u], -du * wo[u]);
@@ -1336,7 +1344,7 @@ __global__ void __launch_bounds__(32 * kStack, U == 8 ? 2 : 1) icd_lockstep_kern
                     hi = cb + mid;
                     lo = cb + b - n1;
                 }
-                off = s * P.nch * P.nr;
+                off = s * (1 << P.rb);
             }
             const int chunks = (n + 32 * U - 1) / (32 * U);
             if (lane == 0) s_chunks[wid] = chunks;
@@ -1444,7 +1452,7 @@ __device__ __forceinline__ void staged_item(const GParams& P, const uint32_t* __
         const int vs = min(max(start[kl] - s, v0), v1);
         mid = cb + vp[vs];
     }
-    const int off = s * P.nch * P.nr;
+    const int off = s * (1 << P.rb);
     const int64_t n1 = en - mid, n = en - b;
 
     float acc_b = 0.f, acc_a = 0.f;
@@ -1555,7 +1563,7 @@ __global__ void __launch_bounds__(32 * WPV, 16 / WPV) icd_cta_kernel(GParams P, 
             en = cb + vp[v1];
             mid = P.stack_align ? cb + vp[stack_start_view(P, start, k, s, v0, v1)] : b;
         }
-        const int off = s * P.nch * P.nr;
+        const int off = s * (1 << P.rb);
         // Sweep position p -> entry p + hi for p < n1 ([mid, en)), else p + lo
         // ([b, mid)).
         const int n = (int)(en - b), n1 = (int)(en - mid);
@@ -1809,8 +1817,9 @@ GParams make_params(const ctbb_recon* rc, const ctbb_ssm* ssm, const ctbb_icd_op
     P.nx = (int)g.num_voxels_x;
     P.ny = (int)g.num_voxels_y;
     P.nz = (int)g.num_voxels_z;
-    P.nch = (int)g.n_channels;
-    P.nr = (int)g.Nrows_projection;
+    P.rb = rc->lay.rb;
+    P.row_mask = rc->lay.row_mask();
+    P.row_step = rc->lay.row_step();
     P.nvsm = (int)ssm->nvsm;
     P.nvsm1 = ssm->nvsm + 1;
     P.readings = (int)g.Readings;
@@ -2587,6 +2596,14 @@ extern "C" ctbb_status ctbb_gpu_batch_iterate(ctbb_batch* b, const ctbb_icd_opts
                     : std::max(4, std::min(b->ctx->sm_count * 32, (int)(0.4 * n_sum / (3.2 * nx_max))));
     bool orders_changed = b->d_merged == nullptr || b->merged_T.size() != b->recons.size();
     std::vector<int> T(b->recons.size());
+    // Scans that share a matrix settle on one layout: a first pass may move the
+    // matrix to a longer scan's, the second moves the shorter scans to it.
+    for (int pass = 0; pass < 2; ++pass)
+        for (size_t i = 0; i < b->recons.size(); ++i) {
+            const bool moved = !(b->recons[i]->lay == b->ssms[i]->lay);
+            CTBB_TRY(match_layout(b->recons[i], b->ssms[i]));
+            if (moved) drop_graph(b);
+        }
     for (size_t i = 0; i < b->recons.size(); ++i) {
         ctbb_recon* rc = b->recons[i];
         const ctbb_ssm* s = b->ssms[i];
