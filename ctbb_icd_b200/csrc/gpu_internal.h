@@ -47,46 +47,53 @@ struct ctbb_ctx {
 };
 
 // Layout of sinograms on the device (error sinogram, FP64 estimate) and of the
-// matrix's sinogram indices: views fastest but for groups of 2^rb detector rows,
-//   ((channel * nrb + (row >> rb)) * stride + view) << rb | row low bits.
-// What bounds the kernels that read it is not bytes but requests: a voxel meets
-// one or two channels and two rows per view, and its channel drifts slowly from
-// view to view, so in the raw data's order (row fastest) neighbouring entries each
-// lie in another 128-byte line. Here a line holds 8 views of 4 rows: the 16 entry
-// pairs of a warp's load touch 6.3 lines instead of 15.5 and 13.7 sectors instead
-// of 17 (512 x 512 x 64 benchmark; 9.6 and 14 on 2.3 mm voxels). A slice's first
-// view still adds a constant (s << rb) to every index of a column, which a blocked
-// order with view blocks does not give. Rows are padded to whole groups, views to
-// whole lines; padding holds zeros. Where that would not fit a 31-bit index, rb
-// is 0 and nothing is padded.
+// matrix's sinogram indices: views fastest but for groups of 2^cb channels x 2^rb
+// detector rows (2 x 2),
+//   ((channel >> cb) * nrb + (row >> rb)) * stride + view, then the channel's and
+//   the row's low bits.
+// What bounds the kernels that read it is not bytes but requests: a voxel meets a
+// few neighbouring channels and two rows per view, and its channels drift slowly
+// from view to view, so in the raw data's order (row fastest) neighbouring entries
+// each lie in another 128-byte line. Here a line holds 8 views of a group and a
+// 32-byte sector two: the 16 entry pairs of a warp's load touch 5.3 lines and 13.3
+// sectors instead of 15.5 and 17 (512 x 512 x 64 benchmark; 6.9 and 10.3 on 2.3 mm
+// voxels; groups of 4 rows of one channel: 5.4 and 13.8, 9.7 and 14.3). A slice's
+// first view still adds a constant (s << shift()) to every index of a column.
+// Channels and rows are padded to whole groups, views to whole lines; padding
+// holds zeros. Where that would not fit a 31-bit index, nothing is grouped.
 struct SinoLayout {
-    int rb = 0, nr = 0, nch = 0, nrb = 0;
+    int rb = 0, cb = 0, nr = 0, nch = 0, nrb = 0, ncb = 0;
     uint32_t stride = 0;  // views, padded
 
     static SinoLayout make(uint64_t nch, uint64_t nr, uint64_t views) {
         SinoLayout l;
         l.nr = (int)nr;
         l.nch = (int)nch;
-        l.rb = nr >= 3 ? 2 : (int)nr - 1;
-        l.nrb = (l.nr + (1 << l.rb) - 1) >> l.rb;
+        l.rb = nr >= 2 ? 1 : 0;
+        l.cb = nch >= 2 ? 1 : 0;
+        l.nrb = (l.nr + l.rb) >> l.rb;
+        l.ncb = (l.nch + l.cb) >> l.cb;
         l.stride = (uint32_t)((views + 7) / 8 * 8);
         if (l.size() >= 2147483648ull) {
-            l.rb = 0;
+            l.rb = l.cb = 0;
             l.nrb = l.nr;
+            l.ncb = l.nch;
             l.stride = (uint32_t)views;
         }
         return l;
     }
-    uint64_t size() const { return ((uint64_t)nch * nrb * stride) << rb; }
+    __host__ __device__ int shift() const { return rb + cb; }
+    uint64_t size() const { return ((uint64_t)ncb * nrb * stride) << (rb + cb); }
     __host__ __device__ uint32_t at(uint32_t view, uint32_t ch, uint32_t row) const {
-        return (((ch * (uint32_t)nrb + (row >> rb)) * stride + view) << rb) | (row & ((1u << rb) - 1u));
+        return ((((ch >> cb) * (uint32_t)nrb + (row >> rb)) * stride + view) << (rb + cb)) |
+               ((ch & (uint32_t)cb) << rb) | (row & (uint32_t)rb);
     }
-    // The inverse; rows and views of the padding come out past the end.
+    // The inverse; rows, channels and views of the padding come out past the end.
     __host__ __device__ void split(uint32_t a, uint32_t* view, uint32_t* ch, uint32_t* row) const {
-        const uint32_t t = a >> rb, u = t / stride, c = u / (uint32_t)nrb;
+        const uint32_t t = a >> (rb + cb), u = t / stride, c = u / (uint32_t)nrb;
         *view = t - u * stride;
-        *ch = c;
-        *row = ((u - c * (uint32_t)nrb) << rb) | (a & ((1u << rb) - 1u));
+        *ch = (c << cb) | ((a >> rb) & (uint32_t)cb);
+        *row = ((u - c * (uint32_t)nrb) << rb) | (a & (uint32_t)rb);
     }
     // The raw data's order (row fastest).
     __host__ __device__ uint32_t linear(uint32_t a) const {
@@ -99,11 +106,13 @@ struct SinoLayout {
         return at(v, t - v * (uint32_t)nch, q - t * (uint32_t)nr);
     }
     // What leads from a row to the next one of the same view and channel: 1 within
-    // a group, row_step() from its last row (low bits all ones) to the next group.
-    __host__ __device__ uint32_t row_mask() const { return (1u << rb) - 1u; }
-    __host__ __device__ uint32_t row_step() const { return (stride << rb) - row_mask(); }
+    // a group, row_step() from its last row (low bit set) to the next group.
+    __host__ __device__ uint32_t row_mask() const { return (uint32_t)rb; }
+    __host__ __device__ uint32_t row_step() const { return (stride << (rb + cb)) - (uint32_t)rb; }
+    // Elements of one channel group: an index's quotient by it tells the group.
+    __host__ __device__ uint32_t plane() const { return ((uint32_t)nrb * stride) << (rb + cb); }
     bool operator==(const SinoLayout& o) const {
-        return rb == o.rb && nr == o.nr && nch == o.nch && stride == o.stride;
+        return rb == o.rb && cb == o.cb && nr == o.nr && nch == o.nch && stride == o.stride;
     }
 };
 

@@ -61,8 +61,11 @@ namespace {
 
 struct GParams {
     int nx, ny, nz, nvsm, readings, penalty;
-    int rb;                    // sinogram layout: a slice's first view adds s << rb to its indices,
-    uint32_t row_mask, row_step;  // and the next detector row is 1 or row_step further (SinoLayout)
+    // Sinogram layout (SinoLayout): a slice's first view adds s << view_shift to its
+    // indices; the next detector row is 1 or, where the row_mask bits are set,
+    // row_step further.
+    int view_shift;
+    uint32_t row_mask, row_step;
     int last_slice[2];  // last slice of each parity
     uint64_t n_items, nvsm1;
     double lambda, delta;
@@ -460,7 +463,7 @@ __device__ __forceinline__ void process_item(const GParams& P, const uint32_t* _
         const int vs = min(max(start[kl] - s, v0), v1);
         mid = cb + vp[vs];
     }
-    const int off = s * (1 << P.rb);
+    const int off = s * (1 << P.view_shift);
 
     // beta = sum a e, alpha = sum a^2 (FP32 accumulation per lane) over
     // [mid, en) then [b, mid).
@@ -642,7 +645,7 @@ __global__ void __launch_bounds__(256) icd_grouped_pairs_kernel(
             mid = cb + vp[min(max(start[kl] - s, v0), v1)];
             n_entries = (int64_t)vptr[col * P.nvsm1 + v1] - (int64_t)vptr[col * P.nvsm1 + v0];
         }
-        const int off = s * (1 << P.rb);
+        const int off = s * (1 << P.view_shift);
         float acc_b = 0.f, acc_a = 0.f;
         const uint64_t keep = l2_keep();
         gather_pairs<U>(P, pairs, e, mid, en, off, lane, keep, acc_b, acc_a);
@@ -731,7 +734,7 @@ __global__ void __launch_bounds__(32 * WPV, 16 / WPV) icd_cta_pairs_kernel(
             mid = P.stack_align ? cb + vp[stack_start_view(P, start, k, s, v0, v1)] : b;
             if (tid == 0) n_entries = (int64_t)vptr[col * P.nvsm1 + v1] - (int64_t)vptr[col * P.nvsm1 + v0];
         }
-        const int off = s * (1 << P.rb);
+        const int off = s * (1 << P.view_shift);
         // Sweep position p (pairs) -> pair p + hi for p < n1 ([mid, en)), else
         // p + lo ([b, mid)).
         const int n = (int)(en - b), n1 = (int)(en - mid);
@@ -922,7 +925,7 @@ __device__ __forceinline__ void bulk_issue(const GParams& P, const uint32_t* __r
     it->en = en;
     it->q = (int64_t)col + (int64_t)ncol * k;
     it->n_entries = ne;
-    it->off = s * (1 << P.rb);
+    it->off = s * (1 << P.view_shift);
     it->d = (int)(b - b0);
     it->ns = ns;
     it->valid = 1;
@@ -1127,7 +1130,7 @@ __device__ __forceinline__ void bulk_claim(const GParams& P, const uint32_t* __r
     it->en = en;
     it->q = (int64_t)col + (int64_t)ncol * k;
     it->n_entries = ne;
-    it->off = s * (1 << P.rb);
+    it->off = s * (1 << P.view_shift);
     it->d = (int)(b - (b & ~(int64_t)1));
     it->ns = ns;
     it->valid = 1;
@@ -1344,7 +1347,7 @@ __global__ void __launch_bounds__(32 * kStack, U == 8 ? 2 : 1) icd_lockstep_kern
                     hi = cb + mid;
                     lo = cb + b - n1;
                 }
-                off = s * (1 << P.rb);
+                off = s * (1 << P.view_shift);
             }
             const int chunks = (n + 32 * U - 1) / (32 * U);
             if (lane == 0) s_chunks[wid] = chunks;
@@ -1452,7 +1455,7 @@ __device__ __forceinline__ void staged_item(const GParams& P, const uint32_t* __
         const int vs = min(max(start[kl] - s, v0), v1);
         mid = cb + vp[vs];
     }
-    const int off = s * (1 << P.rb);
+    const int off = s * (1 << P.view_shift);
     const int64_t n1 = en - mid, n = en - b;
 
     float acc_b = 0.f, acc_a = 0.f;
@@ -1563,7 +1566,7 @@ __global__ void __launch_bounds__(32 * WPV, 16 / WPV) icd_cta_kernel(GParams P, 
             en = cb + vp[v1];
             mid = P.stack_align ? cb + vp[stack_start_view(P, start, k, s, v0, v1)] : b;
         }
-        const int off = s * (1 << P.rb);
+        const int off = s * (1 << P.view_shift);
         // Sweep position p -> entry p + hi for p < n1 ([mid, en)), else p + lo
         // ([b, mid)).
         const int n = (int)(en - b), n1 = (int)(en - mid);
@@ -1817,7 +1820,7 @@ GParams make_params(const ctbb_recon* rc, const ctbb_ssm* ssm, const ctbb_icd_op
     P.nx = (int)g.num_voxels_x;
     P.ny = (int)g.num_voxels_y;
     P.nz = (int)g.num_voxels_z;
-    P.rb = rc->lay.rb;
+    P.view_shift = rc->lay.shift();
     P.row_mask = rc->lay.row_mask();
     P.row_step = rc->lay.row_step();
     P.nvsm = (int)ssm->nvsm;

@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(32 * kSeqWarps) icd_seq_kernel(
     };
     // The first kSeqR entries of each lane: sinogram index (-1: none) and weight.
     auto fetch = [&](int64_t b, int64_t e, int s, int* qi, float* wi) {
-        const uint32_t off = (uint32_t)((int64_t)s << P.lay.rb);  // modulo 2^32: the sum is in range
+        const uint32_t off = (uint32_t)((int64_t)s << P.lay.shift());  // modulo 2^32: the sum is in range
 #pragma unroll
         for (int r = 0; r < kSeqR; ++r) {
             const int64_t m = b + lane + 32 * r;
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(32 * kSeqWarps) icd_seq_kernel(
             alpha += (double)ww;
             beta += (double)wi[r] * ((double)rv[r] - ev[r]);
         }
-        const uint32_t off = (uint32_t)((int64_t)s0 << P.lay.rb);
+        const uint32_t off = (uint32_t)((int64_t)s0 << P.lay.shift());
         for (int64_t m = b + 32 * kSeqR + lane; m < e; m += 32) {
             const float wm = __ldg(w + m);
             const uint32_t index = (uint32_t)__ldg(idx + m) + off;

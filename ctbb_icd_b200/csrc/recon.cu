@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(256) forward_f64_kernel(FpParams P, const int6
         if (v1 <= v0) continue;
         const int64_t cb = colptr[col];
         const int64_t b = cb + vptr[col * P.nvsm1 + v0], e = cb + vptr[col * P.nvsm1 + v1];
-        double* const a = acc + ((int64_t)s << P.lay.rb);
+        double* const a = acc + ((int64_t)s << P.lay.shift());
         for (int64_t m = b + lane; m < e; m += 32) {
             const double w = w32 ? (double)w32[m] : (double)__half2float(w16[m]);
             atomicAdd(a + (uint32_t)idx[m], xv * w);
@@ -53,11 +53,11 @@ __global__ void __launch_bounds__(256) forward_f64_kernel(FpParams P, const int6
     }
 }
 
-// Walk of a sinogram in the device layout beside the raw data: a warp takes 8
-// views x 4 row groups of a channel, so it reads 64-byte runs of the raw rows and
-// writes whole lines. Unit u of the walk for this lane: the element of its group's
-// first row (SINO_END past the sinogram) and the raw index of that row (-1 where the
-// group is padding); rows of the group past the detector are the caller's to skip.
+// Walk of a sinogram in the device layout beside the raw data: a warp takes 4
+// views x 8 row groups of a channel group, a lane one group (4 consecutive
+// elements at most), so both sides move in 64-byte runs. at() gives the group's
+// first element (SINO_END past the sinogram), raw() the raw index of its element k
+// (-1: padding).
 constexpr uint32_t SINO_END = 0xffffffffu;
 struct SinoWalk {
     SinoLayout l;
@@ -67,45 +67,52 @@ struct SinoWalk {
         SinoWalk w;
         w.l = l;
         w.views = (int)views;
-        w.vgroups = ((int)l.stride + 7) / 8;
-        w.rgroups = (l.nrb + 3) / 4;
-        w.units = (uint64_t)w.vgroups * l.nch * w.rgroups;
+        w.vgroups = ((int)l.stride + 3) / 4;
+        w.rgroups = (l.nrb + 7) / 8;
+        w.units = (uint64_t)w.vgroups * l.ncb * w.rgroups;
         return w;
     }
-    __device__ __forceinline__ uint32_t at(uint64_t u, int lane, int64_t* raw, int* row) const {
-        const uint32_t rg = (uint32_t)(u % (uint32_t)rgroups);
-        const uint32_t rest = (uint32_t)(u / (uint32_t)rgroups);
-        const uint32_t c = rest % (uint32_t)l.nch, v = rest / (uint32_t)l.nch * 8 + (lane & 7);
-        const uint32_t rblk = rg * 4 + (lane >> 3);
-        if (v >= l.stride || rblk >= (uint32_t)l.nrb) return SINO_END;
-        *row = (int)(rblk << l.rb);
-        *raw = v < (uint32_t)views ? *row + (int64_t)l.nr * (c + (int64_t)l.nch * v) : -1;
-        return ((c * (uint32_t)l.nrb + rblk) * l.stride + v) << l.rb;
+    __device__ __forceinline__ int group() const { return 1 << l.shift(); }
+    __device__ __forceinline__ uint32_t at(uint64_t u, int lane, uint32_t* v, uint32_t* c, uint32_t* r) const {
+        const uint32_t rest = (uint32_t)(u / (uint32_t)rgroups), rg = (uint32_t)(u - (uint64_t)rest * rgroups);
+        const uint32_t vg = rest / (uint32_t)l.ncb, cblk = rest - vg * (uint32_t)l.ncb;
+        const uint32_t rblk = rg * 8 + (lane & 7);
+        *v = vg * 4 + (lane >> 3);
+        if (*v >= l.stride || rblk >= (uint32_t)l.nrb) return SINO_END;
+        *c = cblk << l.cb;
+        *r = rblk << l.rb;
+        return ((cblk * (uint32_t)l.nrb + rblk) * l.stride + *v) << l.shift();
+    }
+    __device__ __forceinline__ int64_t raw(uint32_t v, uint32_t c, uint32_t r, int k) const {
+        c += (uint32_t)(k >> l.rb);
+        r += (uint32_t)(k & l.rb);
+        return v < (uint32_t)views && c < (uint32_t)l.nch && r < (uint32_t)l.nr && k < group()
+                   ? (int64_t)r + (int64_t)l.nr * (c + (int64_t)l.nch * v)
+                   : -1;
     }
 };
 
 // e = y - acc (acc null: e = y) in the device layout, padding zero.
 __global__ void __launch_bounds__(256) residual_kernel(SinoWalk W, const float* __restrict__ raw,
                                                        const double* __restrict__ acc, float* __restrict__ e32) {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, g = W.group();
     const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     for (uint64_t u = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); u < W.units; u += nwarps) {
-        int64_t q = -1;
-        int row = 0;
-        const uint32_t a = W.at(u, lane, &q, &row);
+        uint32_t v = 0, c = 0, r = 0;
+        const uint32_t a = W.at(u, lane, &v, &c, &r);
         if (a == SINO_END) continue;
-        float y[4] = {0.f, 0.f, 0.f, 0.f}, o[4];
-        if (q >= 0 && W.l.rb == 2 && W.l.nr % 4 == 0)
-            *reinterpret_cast<float4*>(y) = __ldg(reinterpret_cast<const float4*>(raw + q));
-        else
+        float y[4], o[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) y[k] = q >= 0 && k < (1 << W.l.rb) && row + k < W.l.nr ? __ldg(raw + q + k) : 0.f;
+        for (int k = 0; k < 4; ++k) {
+            const int64_t q = W.raw(v, c, r, k);
+            y[k] = q >= 0 ? __ldg(raw + q) : 0.f;
+        }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) o[k] = acc && k < (1 << W.l.rb) ? (float)((double)y[k] - acc[a + k]) : y[k];
-        if (W.l.rb == 2) {
+        for (int k = 0; k < 4; ++k) o[k] = acc && k < g ? (float)((double)y[k] - acc[a + k]) : y[k];
+        if (g == 4) {
             *reinterpret_cast<float4*>(e32 + a) = make_float4(o[0], o[1], o[2], o[3]);
         } else {
-            for (int k = 0; k < (1 << W.l.rb); ++k) e32[a + k] = o[k];
+            for (int k = 0; k < g; ++k) e32[a + k] = o[k];
         }
     }
 }
@@ -172,14 +179,14 @@ __global__ void __launch_bounds__(256) sq_diff_kernel(SinoWalk W, const float* _
     const int lane = threadIdx.x & 31;
     const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     for (uint64_t u = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); u < W.units; u += nwarps) {
-        int64_t q = -1;
-        int row = 0;
-        const uint32_t a = W.at(u, lane, &q, &row);
-        if (a == SINO_END || q < 0) continue;
+        uint32_t v = 0, c = 0, r = 0;
+        const uint32_t a = W.at(u, lane, &v, &c, &r);
+        if (a == SINO_END) continue;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            if (k >= (1 << W.l.rb) || row + k >= W.l.nr) continue;
-            const double d = (double)__ldg(raw + q + k) - acc[a + k];
+            const int64_t q = W.raw(v, c, r, k);
+            if (q < 0) continue;
+            const double d = (double)__ldg(raw + q) - acc[a + k];
             s += d * d;
         }
     }

@@ -318,9 +318,10 @@ __global__ void f32_to_f16_kernel(const float* __restrict__ in, __half* __restri
 // both FP16 weights of a run in 8 bytes (4 per entry instead of 6); a lone
 // entry has w1 = 0. One thread per (column, view) cell: pair count, then
 // (after the same per-column / per-matrix scans as the entries) the fill.
+// Whether an index and its row successor lie in the same channel (the last row's
+// successor falls into the next channel group).
 __device__ __forceinline__ bool same_channel(const SinoLayout& l, uint32_t a, uint32_t b) {
-    const uint32_t plane = (uint32_t)l.nrb * l.stride << l.rb;
-    return a / plane == b / plane;
+    return a / l.plane() == b / l.plane();
 }
 
 template <bool FILL>
