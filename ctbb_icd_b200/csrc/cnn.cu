@@ -314,6 +314,18 @@ __global__ void __launch_bounds__(256) conv_wgrad_kernel(Dims d, const __nv_bflo
     }
 }
 
+// Store a voxel's 32 channels as four 16-byte words (two-channel stores put a warp's
+// lanes in 32 different sectors sixteen times over).
+__device__ __forceinline__ void store_channels(__nv_bfloat16* __restrict__ o, const float* v) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        __align__(16) __nv_bfloat162 h[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) h[k] = __floats2bfloat162_rn(v[8 * q + 2 * k], v[8 * q + 2 * k + 1]);
+        reinterpret_cast<uint4*>(o)[q] = *reinterpret_cast<const uint4*>(h);
+    }
+}
+
 __device__ __forceinline__ bool inside(int x, int y, int z, int nx, int ny, int nz) {
     return x >= 0 && x < nx && y >= 0 && y < ny && z >= 0 && z < nz;
 }
@@ -323,7 +335,7 @@ __device__ __forceinline__ bool inside(int x, int y, int z, int nx, int ny, int 
 __global__ void __launch_bounds__(256) conv_in_kernel(int nx, int ny, int nz, const float* __restrict__ x,
                                                       float s_in, const float* __restrict__ w,
                                                       __nv_bfloat16* __restrict__ out) {
-    __shared__ float sw[kTaps * kC + kC];
+    __shared__ __align__(16) float sw[kTaps * kC + kC];
     for (int i = threadIdx.x; i < kTaps * kC + kC; i += blockDim.x) sw[i] = w[i];
     __syncthreads();
     const uint64_t n = (uint64_t)nx * ny * nz;
@@ -337,11 +349,17 @@ __global__ void __launch_bounds__(256) conv_in_kernel(int nx, int ny, int nz, co
             if (!inside(jx, jy, jz, nx, ny, nz)) continue;
             const float xv = s_in * x[((uint64_t)jz * ny + jy) * nx + jx];
 #pragma unroll
-            for (int c = 0; c < kC; ++c) acc[c] = fmaf(xv, sw[t * kC + c], acc[c]);
+            for (int c = 0; c < kC; c += 4) {
+                const float4 wt = *reinterpret_cast<const float4*>(sw + t * kC + c);
+                acc[c] = fmaf(xv, wt.x, acc[c]);
+                acc[c + 1] = fmaf(xv, wt.y, acc[c + 1]);
+                acc[c + 2] = fmaf(xv, wt.z, acc[c + 2]);
+                acc[c + 3] = fmaf(xv, wt.w, acc[c + 3]);
+            }
         }
-        __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(out + v * kC);
 #pragma unroll
-        for (int c = 0; c < kC; c += 2) o[c / 2] = __floats2bfloat162_rn(fmaxf(acc[c], 0.f), fmaxf(acc[c + 1], 0.f));
+        for (int c = 0; c < kC; ++c) acc[c] = fmaxf(acc[c], 0.f);
+        store_channels(out + v * kC, acc);
     }
 }
 
@@ -423,7 +441,7 @@ __global__ void __launch_bounds__(256) weight_sum_kernel(uint64_t n, const float
 __global__ void __launch_bounds__(256) conv_out_bwd_kernel(int nx, int ny, int nz, const float* __restrict__ dout,
                                                            const float* __restrict__ w,
                                                            __nv_bfloat16* __restrict__ g) {
-    __shared__ float sw[kTaps * kC];
+    __shared__ __align__(16) float sw[kTaps * kC];
     for (int i = threadIdx.x; i < kTaps * kC; i += blockDim.x) sw[i] = w[i];
     __syncthreads();
     const uint64_t n = (uint64_t)nx * ny * nz;
@@ -437,11 +455,15 @@ __global__ void __launch_bounds__(256) conv_out_bwd_kernel(int nx, int ny, int n
             if (!inside(jx, jy, jz, nx, ny, nz)) continue;
             const float dv = dout[((uint64_t)jz * ny + jy) * nx + jx];
 #pragma unroll
-            for (int c = 0; c < kC; ++c) acc[c] = fmaf(dv, sw[t * kC + c], acc[c]);
+            for (int c = 0; c < kC; c += 4) {
+                const float4 wt = *reinterpret_cast<const float4*>(sw + t * kC + c);
+                acc[c] = fmaf(dv, wt.x, acc[c]);
+                acc[c + 1] = fmaf(dv, wt.y, acc[c + 1]);
+                acc[c + 2] = fmaf(dv, wt.z, acc[c + 2]);
+                acc[c + 3] = fmaf(dv, wt.w, acc[c + 3]);
+            }
         }
-        __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(g + v * kC);
-#pragma unroll
-        for (int c = 0; c < kC; c += 2) o[c / 2] = __floats2bfloat162_rn(acc[c], acc[c + 1]);
+        store_channels(g + v * kC, acc);
     }
 }
 
