@@ -214,6 +214,8 @@ ctbb_status recon_to_grouped(ctbb_recon* rc, const ctbb_ssm* ssm);
 ctbb_status recon_to_sequential(ctbb_recon* rc, const ctbb_ssm* ssm);
 ctbb_status arranged_raw(ctbb_recon* rc);  // y in the device layout into d_e32
 ctbb_status match_layout(ctbb_recon* rc, const ctbb_ssm* ssm);
+// Refuses a matrix of another geometry or context, then match_layout.
+ctbb_status check_pair(ctbb_recon* rc, const ctbb_ssm* ssm);
 ctbb_status forward_project_f64(ctbb_recon* rc, const ctbb_ssm* ssm, bool from_x32, double* d_out);
 ctbb_status cost_f64(ctbb_recon* rc, const ctbb_ssm* ssm, bool exact, double* out);
 

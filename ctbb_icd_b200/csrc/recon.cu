@@ -264,16 +264,6 @@ FpParams fp_params(const ctbb_recon* rc, const ctbb_ssm* ssm) {
     return P;
 }
 
-ctbb_status check_pair(ctbb_recon* rc, const ctbb_ssm* ssm) {
-    const ctbb_geom_c &a = rc->geom, &b = ssm->geom;
-    if (a.num_voxels_x != b.num_voxels_x || a.num_voxels_y != b.num_voxels_y || a.n_channels != b.n_channels ||
-        a.Nrows_projection != b.Nrows_projection || a.num_views_for_system_matrix != b.num_views_for_system_matrix)
-        return ctbb::fail(CTBB_ERR_INVALID_ARG, "system matrix geometry does not match the reconstruction");
-    if (rc->ctx != ssm->ctx) return ctbb::fail(CTBB_ERR_INVALID_ARG, "matrix and reconstruction use different contexts");
-    CTBB_CUDA(cudaSetDevice(rc->ctx->device));
-    return ctbb::match_layout(rc, ssm);
-}
-
 // e = y - est (or y alone) in the device layout.
 ctbb_status residual(ctbb_recon* rc, const double* est) {
     const SinoWalk W = SinoWalk::make(rc->lay, rc->geom.Readings);
@@ -332,6 +322,16 @@ ctbb_status match_layout(ctbb_recon* rc, const ctbb_ssm* ssm) {
     rc->lay = ssm->lay;
     rc->sino_size = n;
     return CTBB_OK;
+}
+
+ctbb_status check_pair(ctbb_recon* rc, const ctbb_ssm* ssm) {
+    const ctbb_geom_c &a = rc->geom, &b = ssm->geom;
+    if (a.num_voxels_x != b.num_voxels_x || a.num_voxels_y != b.num_voxels_y || a.n_channels != b.n_channels ||
+        a.Nrows_projection != b.Nrows_projection || a.num_views_for_system_matrix != b.num_views_for_system_matrix)
+        return fail(CTBB_ERR_INVALID_ARG, "system matrix geometry does not match the reconstruction");
+    if (rc->ctx != ssm->ctx) return fail(CTBB_ERR_INVALID_ARG, "matrix and reconstruction use different contexts");
+    CTBB_CUDA(cudaSetDevice(rc->ctx->device));
+    return match_layout(rc, ssm);
 }
 
 ctbb_status forward_project_f64(ctbb_recon* rc, const ctbb_ssm* ssm, bool from_x32, double* d_out) {

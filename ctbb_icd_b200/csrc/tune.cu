@@ -26,8 +26,7 @@ extern "C" ctbb_status ctbb_gpu_recon_autotune(ctbb_recon* rc, const ctbb_ssm* s
     if ((wsel == CTBB_SSM_FP32 && !ssm->d_w32) || (wsel == CTBB_SSM_FP16 && !ssm->d_w16))
         return fail(CTBB_ERR_INVALID_ARG, "requested weight format is not held by the matrix");
     o.weights = wsel;
-    CTBB_CUDA(cudaSetDevice(rc->ctx->device));
-    CTBB_TRY(match_layout(rc, ssm));
+    CTBB_TRY(check_pair(rc, ssm));
     CTBB_TRY(recon_to_grouped(rc, ssm));
     CTBB_TRY(ctbb_gpu_recon_refresh_residual(rc, ssm));
     double c0 = 0.0;

@@ -66,3 +66,23 @@ def test_matrix_shared_by_scans_of_different_length(ctx, tmp_path, mode, longer_
         v, cost = run(i, ssm)
         assert np.linalg.norm(v - own[i][0]) <= 1e-5 * np.linalg.norm(own[i][0])
         assert abs(cost - own[i][1]) <= 1e-5 * own[i][1]
+
+
+def test_autotune_refuses_a_matrix_of_another_geometry(ctx, tmp_path):
+    """The refusal comes before the matrix and the scan settle on one layout."""
+    _, rp = W.materialise("small", str(tmp_path / "a"))
+    _, other = W.materialise("tiny", str(tmp_path / "b"))
+    data = C.load_raw(rp)
+    rc = C.Recon(rp, data.slice_indices, ctx)
+    rc.set_raw(data.raw)
+    ssm = C.Ssm.generate(rp, ctx, C.SSM_BOTH)
+    ssm_other = C.Ssm.generate(other, ctx, C.SSM_BOTH)
+    rc.set_volume(ssm, None)
+    mid = int(ssm_other.info().n_columns) // 2
+    before = ssm_other.column(mid)
+    with pytest.raises(C.CtbbError, match="geometry does not match"):
+        rc.autotune(ssm_other, C.icd_opts(mode=C.ICD_GROUPED, weights=C.SSM_FP16))
+    after = ssm_other.column(mid)
+    assert all(np.array_equal(a, b) for a, b in zip(before, after))
+    for o in (rc, ssm, ssm_other):
+        o.free()
