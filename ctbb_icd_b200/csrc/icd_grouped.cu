@@ -687,7 +687,7 @@ __device__ __forceinline__ void load_seq_pairs(const GParams& P, const uint2* __
 // U entries of a lane from a whole chunk of 16 x U pairs: no bounds tests, one
 // pointer. The index lacks the slice's offset, which is in the caller's e pointer;
 // -1: the second entry of a lone one.
-template <int U, int STRIDE = 16>
+template <int U>
 __device__ __forceinline__ void load_whole_pairs(const GParams& P, const uint2* __restrict__ pp, int half, uint64_t pol,
                                                  int* q, float* wt) {
     const int to_next = half ? 1 : 0, to_step = half ? (int)P.row_step : 0;
@@ -696,7 +696,7 @@ __device__ __forceinline__ void load_whole_pairs(const GParams& P, const uint2* 
         uint32_t a, bb;
         asm volatile("ld.global.nc.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;"
                      : "=r"(a), "=r"(bb)
-                     : "l"(pp + STRIDE * u), "l"(pol));
+                     : "l"(pp + 16 * u), "l"(pol));
         const uint32_t wb = half ? bb >> 16 : bb & 0xffffu;
         q[u] = (int)a + ((a & P.row_mask) == P.row_mask ? to_step : to_next);
         wt[u] = __half2float(__ushort_as_half((unsigned short)wb));
@@ -1103,87 +1103,8 @@ __device__ __forceinline__ void bulk_issue(const GParams& P, const uint32_t* __r
     }
 }
 
-// The pairs of a window past the stage, streamed from global memory for the
-// gather and again for the scatter (wide voxels: most of the column). Whole chunks
-// of 1024 pairs carry no bounds tests, and the next chunk's pairs are fetched while
-// this one's e values or reductions are in flight.
-__device__ __forceinline__ void bulk_tail_gather(const GParams& P, const uint2* __restrict__ pairs, const float* e,
-                                                 const BulkItem& it, int n, int j, int half, uint64_t pol, float& acc_b,
-                                                 float& acc_a) {
-    int left = n - it.ns;
-    if (left <= 0) return;
-    const float* const eo = e + it.off;
-    const uint2* pp = pairs + it.b + it.ns + j;
-    int q[kU];
-    float w[kU];
-    if (left >= kBulkNP * kU) load_whole_pairs<kU, kBulkNP>(P, pp, half, pol, q, w);
-    while (left >= kBulkNP * kU) {
-        float ev[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) ev[u] = q[u] != INT_MIN ? __ldcg(eo + q[u]) : 0.f;
-        left -= kBulkNP * kU;
-        pp += kBulkNP * kU;
-        int qn[kU];
-        float wn[kU];
-        if (left >= kBulkNP * kU) load_whole_pairs<kU, kBulkNP>(P, pp, half, pol, qn, wn);
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            acc_b = fmaf(w[u], ev[u], acc_b);
-            acc_a = fmaf(w[u], w[u], acc_a);
-            q[u] = qn[u];
-            w[u] = wn[u];
-        }
-    }
-    if (left > 0) {
-        load_pair_entries<kU, kBulkNP>(P, pairs, it.en - left + j, it.en, it.off, half, pol, q, w);
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const float ev = q[u] >= 0 ? __ldcg(e + q[u]) : 0.f;
-            acc_b = fmaf(w[u], ev, acc_b);
-            acc_a = fmaf(w[u], w[u], acc_a);
-        }
-    }
-}
-
-__device__ __forceinline__ void bulk_tail_scatter(const GParams& P, const uint2* __restrict__ pairs, float* e,
-                                                  const BulkItem& it, int n, int j, int half, uint64_t pol, float du) {
-    int left = n - it.ns;
-    if (left <= 0) return;
-    float* const eo = e + it.off;
-    const uint2* pp = pairs + it.b + it.ns + j;
-    int q[kU];
-    float w[kU];
-    if (left >= kBulkNP * kU) load_whole_pairs<kU, kBulkNP>(P, pp, half, pol, q, w);
-    while (left >= kBulkNP * kU) {
-        left -= kBulkNP * kU;
-        pp += kBulkNP * kU;
-        int qn[kU];
-        float wn[kU];
-        if (left >= kBulkNP * kU) load_whole_pairs<kU, kBulkNP>(P, pp, half, pol, qn, wn);
-#pragma unroll
-        for (int u = 0; u < kU; ++u)
-            if (q[u] != INT_MIN) atomicAdd(eo + q[u], -du * w[u]);
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            q[u] = qn[u];
-            w[u] = wn[u];
-        }
-    }
-    if (left > 0) {
-        load_pair_entries<kU, kBulkNP>(P, pairs, it.en - left + j, it.en, it.off, half, pol, q, w);
-#pragma unroll
-        for (int u = 0; u < kU; ++u)
-            if (q[u] >= 0) atomicAdd(e + q[u], -du * w[u]);
-    }
-}
-
-// LONG: two CTAs per SM at most, so that the prefetching tail fits in registers; for
-// columns mostly past the stage, whose updates in flight are few (128 x 128 x 16 at
-// 2.3 mm, 15 k pairs a column, 32 in flight: 500 -> 220 ms an iteration). The plain
-// tail keeps four CTAs per SM for short columns (with the long one inlined,
-// 512 x 512 x 64 spilled and took 524 ms instead of 482).
-template <int STAGES, bool LONG>
-__global__ void __launch_bounds__(kBulkThreads, LONG ? 2 : STAGES == 1 ? 4 : 3) icd_bulk_kernel(
+template <int STAGES>
+__global__ void __launch_bounds__(kBulkThreads, STAGES == 1 ? 4 : 3) icd_bulk_kernel(
     GParams P, const uint32_t* __restrict__ order, const int64_t* __restrict__ pcolptr,
     const uint32_t* __restrict__ pvptr, const uint2* __restrict__ pairs, const uint32_t* __restrict__ vptr,
     const int32_t* __restrict__ start, float* e, float* x, unsigned long long* queue, unsigned long long* stats,
@@ -1250,19 +1171,15 @@ __global__ void __launch_bounds__(kBulkThreads, LONG ? 2 : STAGES == 1 ? 4 : 3) 
                 acc_a = fmaf(wv, wv, acc_a);
             }
         }
-        if (LONG) {
-            bulk_tail_gather(P, pairs, e, it, n, j, half, pol, acc_b, acc_a);
-        } else {
-            for (int b2 = it.ns; b2 < n; b2 += kBulkNP * kU) {
-                int qo[kU];
-                float wo[kU];
-                load_pair_entries<kU, kBulkNP>(P, pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
+        for (int b2 = it.ns; b2 < n; b2 += kBulkNP * kU) {
+            int qo[kU];
+            float wo[kU];
+            load_pair_entries<kU, kBulkNP>(P, pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
 #pragma unroll
-                for (int u = 0; u < kU; ++u) {
-                    const float evu = qo[u] >= 0 ? __ldcg(e + qo[u]) : 0.f;
-                    acc_b = fmaf(wo[u], evu, acc_b);
-                    acc_a = fmaf(wo[u], wo[u], acc_a);
-                }
+            for (int u = 0; u < kU; ++u) {
+                const float evu = qo[u] >= 0 ? __ldcg(e + qo[u]) : 0.f;
+                acc_b = fmaf(wo[u], evu, acc_b);
+                acc_a = fmaf(wo[u], wo[u], acc_a);
             }
         }
         acc_b = warp_sum(acc_b);
@@ -1300,17 +1217,13 @@ __global__ void __launch_bounds__(kBulkThreads, LONG ? 2 : STAGES == 1 ? 4 : 3) 
                         atomicAdd(e + pair_index(P, pr.x, it.off, half), -du * (half ? half_hi(pr.y) : half_lo(pr.y)));
                 }
             }
-            if (LONG) {
-                bulk_tail_scatter(P, pairs, e, it, n, j, half, pol, du);
-            } else {
-                for (int b2 = it.ns; b2 < n; b2 += kBulkNP * kU) {
-                    int qo[kU];
-                    float wo[kU];
-                    load_pair_entries<kU, kBulkNP>(P, pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
+            for (int b2 = it.ns; b2 < n; b2 += kBulkNP * kU) {
+                int qo[kU];
+                float wo[kU];
+                load_pair_entries<kU, kBulkNP>(P, pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
 #pragma unroll
-                    for (int u = 0; u < kU; ++u)
-                        if (qo[u] >= 0) atomicAdd(e + qo[u], -du * wo[u]);
-                }
+                for (int u = 0; u < kU; ++u)
+                    if (qo[u] >= 0) atomicAdd(e + qo[u], -du * wo[u]);
             }
             n_ent += (unsigned long long)it.n_entries;
             ++n_upd;
@@ -2468,25 +2381,23 @@ ctbb_status launch_icd_grouped(ctbb_recon* rc, const ctbb_ssm* ssm, const ctbb_i
         if (stage >= 4) {
             // One update per CTA of 8 warps; 4: one pair stage, 5: two.
             const int stages = stage == 4 ? 1 : 2;
-            const bool long_columns =
-                in_flight <= 2 * (uint64_t)ctx->sm_count && 2 * ssm->npairs > 3 * (uint64_t)kBulkCap * ssm->ncol;
             const size_t smem = bulk_smem_bytes(stages);
             if (prepare) {
                 if (stages == 1)
-                    CTBB_CUDA(cudaFuncSetAttribute(long_columns ? icd_bulk_kernel<1, true> : icd_bulk_kernel<1, false>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                    CTBB_CUDA(cudaFuncSetAttribute(icd_bulk_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)smem));
                 else
-                    CTBB_CUDA(cudaFuncSetAttribute(icd_bulk_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                    CTBB_CUDA(cudaFuncSetAttribute(icd_bulk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int)smem));
                 return CTBB_OK;
             }
             const int blocks = (int)std::max<uint64_t>(1, in_flight);
             if (stages == 1)
-                (long_columns ? icd_bulk_kernel<1, true> : icd_bulk_kernel<1, false>)<<<blocks, kBulkThreads, smem, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr,
+                icd_bulk_kernel<1><<<blocks, kBulkThreads, smem, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr,
                                                                       ssm->d_pairs, vp, rc->d_start, rc->d_e32,
                                                                       rc->d_x32, ctx->d_queue, stats, stats + 2);
             else
-                icd_bulk_kernel<2, false><<<blocks, kBulkThreads, smem, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr,
+                icd_bulk_kernel<2><<<blocks, kBulkThreads, smem, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr,
                                                                       ssm->d_pairs, vp, rc->d_start, rc->d_e32,
                                                                       rc->d_x32, ctx->d_queue, stats, stats + 2);
             CTBB_CUDA(cudaGetLastError());
