@@ -45,7 +45,6 @@
 // The warp count in flight bounds how stale a gather can be: with W warps
 // and a voxel footprint crossing ~T voxels per ray, about T*W/N voxels of a
 // ray change concurrently; the default keeps that near 0.4.
-#include <limits.h>
 #include <math.h>
 
 #include <string.h>
@@ -135,6 +134,24 @@ __device__ __forceinline__ float ldw_hint<__half>(const __half* w, int64_t m, ui
     return __half2float(__ushort_as_half(v));
 }
 
+// Entries m, m+32, ..., m+32(U-1) of a column: sinogram index (q + off, or
+// -1 past the end) and weight (0 past the end).
+template <int U, class WT>
+__device__ __forceinline__ void load_chunk(const int32_t* __restrict__ idx, const WT* __restrict__ w, int64_t m,
+                                           int64_t en, int off, uint64_t pol, int* q, float* wt) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int64_t mu = m + 32 * u;
+        if (mu < en) {
+            q[u] = ld_idx(idx + mu, pol) + off;
+            wt[u] = ldw_hint(w, mu, pol);
+        } else {
+            q[u] = -1;
+            wt[u] = 0.f;
+        }
+    }
+}
+
 // Sinogram index of a pair's entry: the pair's own row a, or the next one.
 __device__ __forceinline__ int pair_index(const GParams& P, uint32_t a, int off, int half) {
     const uint32_t step = (a & P.row_mask) == P.row_mask ? P.row_step : 1u;
@@ -159,134 +176,11 @@ __device__ __forceinline__ int stack_start_view(const GParams& P, const int32_t*
     return min(max(start[kl] - s, v0), v1);
 }
 
-// U entries of a lane from a chunk of 32 x U: whole chunks load at immediate
-// offsets from one pointer, the last one only the entries below n (the others get
-// weight 0 and are not valid).
-template <int U, class WT>
-__device__ __forceinline__ void load_whole(const int32_t* __restrict__ ip, const WT* __restrict__ wp, uint64_t pol,
-                                           int* q, float* wt) {
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        q[u] = ld_idx(ip + 32 * u, pol);
-        wt[u] = ldw_hint(wp, 32 * u, pol);
-    }
-}
-
 // Gather beta += a e and alpha += a^2 over entries [b, en) of a column: chunks
 // of 32 x U entries, the next chunk's indices and weights fetched while this
-// chunk's e gathers are in flight (one DRAM round trip per chunk). With few warps on
-// an SM the chain is the warp's own instruction issue, so whole chunks carry no
-// bounds tests and no address arithmetic but one wide multiply-add per gather.
+// chunk's e gathers are in flight (one DRAM round trip per chunk).
 template <class WT, int U>
 __device__ __forceinline__ void gather_range(const int32_t* __restrict__ idx, const WT* __restrict__ w,
-                                             const float* e, int64_t b, int64_t en, int off, int lane,
-                                             uint64_t pol, float& acc_b, float& acc_a) {
-    if (b >= en) return;
-    const float* const eo = e + off;
-    const int32_t* ip = idx + b + lane;
-    const WT* wp = w + b + lane;
-    int left = (int)(en - b);
-    int qa[U];
-    float wa[U];
-    if (left >= 32 * U) load_whole<U>(ip, wp, pol, qa, wa);
-    while (left >= 32 * U) {
-        float ev[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) ev[u] = __ldcg(eo + qa[u]);
-        left -= 32 * U;
-        ip += 32 * U;
-        wp += 32 * U;
-        int qb[U];
-        float wb[U];
-        if (left >= 32 * U) load_whole<U>(ip, wp, pol, qb, wb);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            acc_b = fmaf(wa[u], ev[u], acc_b);
-            acc_a = fmaf(wa[u], wa[u], acc_a);
-            qa[u] = qb[u];
-            wa[u] = wb[u];
-        }
-    }
-    if (left > 0) {
-        float ev[U], wt[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            ev[u] = wt[u] = 0.f;
-            if (lane + 32 * u < left) {
-                wt[u] = ldw_hint(wp, 32 * u, pol);
-                ev[u] = __ldcg(eo + ld_idx(ip + 32 * u, pol));
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            acc_b = fmaf(wt[u], ev[u], acc_b);
-            acc_a = fmaf(wt[u], wt[u], acc_a);
-        }
-    }
-}
-
-// e -= du * a over entries [b, en): U independent index/weight loads per
-// lane per chunk, then U fire-and-forget L2 reductions. Chunks run from the
-// end of the range back to its start: the entries gathered last are the ones
-// whose matrix lines and e sectors are likeliest to still be in L2.
-template <class WT, int U>
-__device__ __forceinline__ void scatter_range(const int32_t* __restrict__ idx, const WT* __restrict__ w, float* e,
-                                              int64_t b, int64_t en, int off, int lane, uint64_t pol, float du) {
-    if (b >= en) return;
-    float* const eo = e + off;
-    const int n = (int)(en - b), whole = n / (32 * U);
-    const int32_t* ip = idx + b + lane + (int64_t)whole * (32 * U);
-    const WT* wp = w + b + lane + (int64_t)whole * (32 * U);
-    const int left = n - whole * (32 * U);
-    if (left > 0) {
-        int q[U];
-        float wt[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (lane + 32 * u < left) {
-                q[u] = ld_idx(ip + 32 * u, pol);
-                wt[u] = ldw_hint(wp, 32 * u, pol);
-            }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (lane + 32 * u < left) atomicAdd(eo + q[u], -du * wt[u]);
-    }
-    for (int c = 0; c < whole; ++c) {
-        ip -= 32 * U;
-        wp -= 32 * U;
-        int q[U];
-        float wt[U];
-        load_whole<U>(ip, wp, pol, q, wt);
-#pragma unroll
-        for (int u = 0; u < U; ++u) atomicAdd(eo + q[u], -du * wt[u]);
-    }
-}
-
-// Entries m, m+32, ..., m+32(U-1) of a column: sinogram index (q + off, or
-// -1 past the end) and weight (0 past the end).
-template <int U, class WT>
-__device__ __forceinline__ void load_chunk(const int32_t* __restrict__ idx, const WT* __restrict__ w, int64_t m,
-                                           int64_t en, int off, uint64_t pol, int* q, float* wt) {
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const int64_t mu = m + 32 * u;
-        if (mu < en) {
-            q[u] = ld_idx(idx + mu, pol) + off;
-            wt[u] = ldw_hint(w, mu, pol);
-        } else {
-            q[u] = -1;
-            wt[u] = 0.f;
-        }
-    }
-}
-
-// The same with every entry bounds-checked. The batched kernel keeps it: there the
-// scatter's matrix loads miss L2 (several matrices share it), so whole chunks
-// shorten its gather but not its scatter (162 -> 107 ms an iteration of four
-// scans), and with that other pace of reading and writing e its iterates leave
-// the run-to-run spread of the checked ones by two to three times.
-template <class WT, int U>
-__device__ __forceinline__ void gather_checked(const int32_t* __restrict__ idx, const WT* __restrict__ w,
                                              const float* e, int64_t b, int64_t en, int off, int lane,
                                              uint64_t pol, float& acc_b, float& acc_a) {
     if (b >= en) return;
@@ -310,8 +204,12 @@ __device__ __forceinline__ void gather_checked(const int32_t* __restrict__ idx, 
     }
 }
 
+// e -= du * a over entries [b, en): U independent index/weight loads per
+// lane per chunk, then U fire-and-forget L2 reductions. Chunks run from the
+// end of the range back to its start: the entries gathered last are the ones
+// whose matrix lines and e sectors are likeliest to still be in L2.
 template <class WT, int U>
-__device__ __forceinline__ void scatter_checked(const int32_t* __restrict__ idx, const WT* __restrict__ w, float* e,
+__device__ __forceinline__ void scatter_range(const int32_t* __restrict__ idx, const WT* __restrict__ w, float* e,
                                               int64_t b, int64_t en, int off, int lane, uint64_t pol, float du) {
     if (b >= en) return;
     const int64_t nchunk = (en - b + 32 * U - 1) / (32 * U);
@@ -538,7 +436,7 @@ __global__ void __launch_bounds__(256) penalty_steps_kernel(int penalty, double 
 }
 
 // One voxel update (work item `item` of a scan's visiting order) by one warp.
-template <class WT, int U = kU, bool CHECKED = false>
+template <class WT, int U = kU>
 __device__ __forceinline__ void process_item(const GParams& P, const uint32_t* __restrict__ order,
                                              const int64_t* __restrict__ colptr, const uint32_t* __restrict__ vptr,
                                              const int32_t* __restrict__ idx, const WT* __restrict__ w,
@@ -571,13 +469,8 @@ __device__ __forceinline__ void process_item(const GParams& P, const uint32_t* _
     // [mid, en) then [b, mid).
     float acc_b = 0.f, acc_a = 0.f;
     const uint64_t keep = l2_keep();
-    if (CHECKED) {
-        gather_checked<WT, U>(idx, w, e, mid, en, off, lane, keep, acc_b, acc_a);
-        gather_checked<WT, U>(idx, w, e, b, mid, off, lane, keep, acc_b, acc_a);
-    } else {
-        gather_range<WT, U>(idx, w, e, mid, en, off, lane, keep, acc_b, acc_a);
-        gather_range<WT, U>(idx, w, e, b, mid, off, lane, keep, acc_b, acc_a);
-    }
+    gather_range<WT, U>(idx, w, e, mid, en, off, lane, keep, acc_b, acc_a);
+    gather_range<WT, U>(idx, w, e, b, mid, off, lane, keep, acc_b, acc_a);
     const double beta = (double)warp_sum(acc_b);
     const double alpha = (double)warp_sum(acc_a);
 
@@ -589,13 +482,8 @@ __device__ __forceinline__ void process_item(const GParams& P, const uint32_t* _
     if (du != 0.f) {
         // Reverse of the gather order: [b, mid) backwards, then [mid, en).
         const uint64_t drop = l2_drop();
-        if (CHECKED) {
-            scatter_checked<WT, U>(idx, w, e, b, mid, off, lane, drop, du);
-            scatter_checked<WT, U>(idx, w, e, mid, en, off, lane, drop, du);
-        } else {
-            scatter_range<WT, U>(idx, w, e, b, mid, off, lane, drop, du);
-            scatter_range<WT, U>(idx, w, e, mid, en, off, lane, drop, du);
-        }
+        scatter_range<WT, U>(idx, w, e, b, mid, off, lane, drop, du);
+        scatter_range<WT, U>(idx, w, e, mid, en, off, lane, drop, du);
         if (scattered) *scattered += (unsigned long long)(en - b);
     }
 }
@@ -684,47 +572,21 @@ __device__ __forceinline__ void load_seq_pairs(const GParams& P, const uint2* __
     }
 }
 
-// U entries of a lane from a whole chunk of 16 x U pairs: no bounds tests, one
-// pointer. The index lacks the slice's offset, which is in the caller's e pointer;
-// -1: the second entry of a lone one.
 template <int U>
-__device__ __forceinline__ void load_whole_pairs(const GParams& P, const uint2* __restrict__ pp, int half, uint64_t pol,
-                                                 int* q, float* wt) {
-    const int to_next = half ? 1 : 0, to_step = half ? (int)P.row_step : 0;
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        uint32_t a, bb;
-        asm volatile("ld.global.nc.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;"
-                     : "=r"(a), "=r"(bb)
-                     : "l"(pp + 16 * u), "l"(pol));
-        const uint32_t wb = half ? bb >> 16 : bb & 0xffffu;
-        q[u] = (int)a + ((a & P.row_mask) == P.row_mask ? to_step : to_next);
-        wt[u] = __half2float(__ushort_as_half((unsigned short)wb));
-        if (half && wb == 0) q[u] = INT_MIN;
-    }
-}
-
-template <int U>
-__device__ __forceinline__ void gather_pairs(const GParams& P, const uint2* __restrict__ pairs, const float* e,
-                                             int64_t b, int64_t en, int off, int lane, uint64_t pol, float& acc_b,
-                                             float& acc_a) {
+__device__ __forceinline__ void gather_pairs(const GParams& P, const uint2* __restrict__ pairs, const float* e, int64_t b, int64_t en,
+                                             int off, int lane, uint64_t pol, float& acc_b, float& acc_a) {
     if (b >= en) return;
     const int half = lane & 1, j = lane >> 1;
-    const float* const eo = e + off;
-    const uint2* pp = pairs + b + j;
-    int left = (int)(en - b);
     int qa[U];
     float wa[U];
-    if (left >= 16 * U) load_whole_pairs<U>(P, pp, half, pol, qa, wa);
-    while (left >= 16 * U) {
+    load_pair_entries<U>(P, pairs, b + j, en, off, half, pol, qa, wa);
+    for (int64_t base = b; base < en; base += 16 * U) {
         float ev[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) ev[u] = qa[u] != INT_MIN ? __ldcg(eo + qa[u]) : 0.f;
-        left -= 16 * U;
-        pp += 16 * U;
+        for (int u = 0; u < U; ++u) ev[u] = qa[u] >= 0 ? __ldcg(e + qa[u]) : 0.f;
         int qb[U];
         float wb[U];
-        if (left >= 16 * U) load_whole_pairs<U>(P, pp, half, pol, qb, wb);
+        load_pair_entries<U>(P, pairs, base + 16 * U + j, en, off, half, pol, qb, wb);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             acc_b = fmaf(wa[u], ev[u], acc_b);
@@ -733,41 +595,21 @@ __device__ __forceinline__ void gather_pairs(const GParams& P, const uint2* __re
             wa[u] = wb[u];
         }
     }
-    if (left > 0) {
-        load_pair_entries<U>(P, pairs, en - left + j, en, off, half, pol, qa, wa);
-        float ev[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) ev[u] = qa[u] >= 0 ? __ldcg(e + qa[u]) : 0.f;
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            acc_b = fmaf(wa[u], ev[u], acc_b);
-            acc_a = fmaf(wa[u], wa[u], acc_a);
-        }
-    }
 }
 
 template <int U>
-__device__ __forceinline__ void scatter_pairs(const GParams& P, const uint2* __restrict__ pairs, float* e, int64_t b,
-                                              int64_t en, int off, int lane, uint64_t pol, float du) {
+__device__ __forceinline__ void scatter_pairs(const GParams& P, const uint2* __restrict__ pairs, float* e, int64_t b, int64_t en,
+                                              int off, int lane, uint64_t pol, float du) {
     if (b >= en) return;
     const int half = lane & 1, j = lane >> 1;
-    float* const eo = e + off;
-    const int n = (int)(en - b), whole = n / (16 * U);
-    const uint2* pp = pairs + b + j + (int64_t)whole * (16 * U);
-    int q[U];
-    float wt[U];
-    if (n > whole * (16 * U)) {
-        load_pair_entries<U>(P, pairs, b + (int64_t)whole * (16 * U) + j, en, off, half, pol, q, wt);
+    const int64_t nchunk = (en - b + 16 * U - 1) / (16 * U);
+    for (int64_t c = nchunk - 1; c >= 0; --c) {
+        int qs[U];
+        float ws[U];
+        load_pair_entries<U>(P, pairs, b + c * (16 * U) + j, en, off, half, pol, qs, ws);
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (q[u] >= 0) atomicAdd(e + q[u], -du * wt[u]);
-    }
-    for (int c = 0; c < whole; ++c) {
-        pp -= 16 * U;
-        load_whole_pairs<U>(P, pp, half, pol, q, wt);
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (q[u] != INT_MIN) atomicAdd(eo + q[u], -du * wt[u]);
+            if (qs[u] >= 0) atomicAdd(e + qs[u], -du * ws[u]);
     }
 }
 
@@ -1834,7 +1676,7 @@ __global__ void __launch_bounds__(256) icd_batch_kernel(const ScanRefs<WT>* __re
         const ScanRefs<WT>& S = scans[m >> 40];
         GParams P = S.P;
         P.relax = relax;
-        process_item<WT, kU, true>(P, S.order, S.colptr, S.vptr, S.idx, S.w, S.start, S.e, S.x, m & ((1ull << 40) - 1), lane);
+        process_item(P, S.order, S.colptr, S.vptr, S.idx, S.w, S.start, S.e, S.x, m & ((1ull << 40) - 1), lane);
     }
 }
 
@@ -2446,38 +2288,31 @@ ctbb_status launch_icd_grouped(ctbb_recon* rc, const ctbb_ssm* ssm, const ctbb_i
                 P, order, ssm, ssm->d_w32, rc, in_flight, stats, s, prepare);
         }
         if (prepare) return CTBB_OK;
-        // One warp per update: in_flight rounded up to 8 warps, in as many CTAs as
-        // there are SMs (8 warps of one CTA share an SM's load/store unit: 128 x 128
-        // x 16, 256 updates in flight, 141 -> 121 ms for two iterations).
-        const int warps = (int)((in_flight + 7) / 8 * 8);
-        int wpc = 8;
-        while (wpc > 1 && warps / wpc < ctx->sm_count) wpc /= 2;
-        const int nthr = 32 * wpc;
         if (wpv == 1 && pairs) {
-            const int blocks = warps / wpc;
+            const int blocks = (int)std::max<uint64_t>(1, (in_flight + 7) / 8);
             if (epl == 16)
-                icd_grouped_pairs_kernel<16><<<blocks, nthr, 0, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr,
+                icd_grouped_pairs_kernel<16><<<blocks, 256, 0, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr,
                                                                     ssm->d_pairs, vp, rc->d_start, rc->d_e32,
                                                                     rc->d_x32, ctx->d_queue, stats);
             else
-                icd_grouped_pairs_kernel<8><<<blocks, nthr, 0, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr,
+                icd_grouped_pairs_kernel<8><<<blocks, 256, 0, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr,
                                                                    ssm->d_pairs, vp, rc->d_start, rc->d_e32,
                                                                    rc->d_x32, ctx->d_queue, stats);
         } else if (wpv == 1) {
-            const int blocks = warps / wpc;
+            const int blocks = (int)std::max<uint64_t>(1, (in_flight + 7) / 8);
             if (epl == 16) {
                 if (h)
-                    icd_grouped_kernel<__half, 16><<<blocks, nthr, 0, s>>>(P, order, cp, vp, ix, ssm->d_w16, rc->d_start,
+                    icd_grouped_kernel<__half, 16><<<blocks, 256, 0, s>>>(P, order, cp, vp, ix, ssm->d_w16, rc->d_start,
                                                                           rc->d_e32, rc->d_x32, ctx->d_queue, stats);
                 else
-                    icd_grouped_kernel<float, 16><<<blocks, nthr, 0, s>>>(P, order, cp, vp, ix, ssm->d_w32, rc->d_start,
+                    icd_grouped_kernel<float, 16><<<blocks, 256, 0, s>>>(P, order, cp, vp, ix, ssm->d_w32, rc->d_start,
                                                                          rc->d_e32, rc->d_x32, ctx->d_queue, stats);
             } else {
                 if (h)
-                    icd_grouped_kernel<__half, 8><<<blocks, nthr, 0, s>>>(P, order, cp, vp, ix, ssm->d_w16, rc->d_start,
+                    icd_grouped_kernel<__half, 8><<<blocks, 256, 0, s>>>(P, order, cp, vp, ix, ssm->d_w16, rc->d_start,
                                                                          rc->d_e32, rc->d_x32, ctx->d_queue, stats);
                 else
-                    icd_grouped_kernel<float, 8><<<blocks, nthr, 0, s>>>(P, order, cp, vp, ix, ssm->d_w32, rc->d_start,
+                    icd_grouped_kernel<float, 8><<<blocks, 256, 0, s>>>(P, order, cp, vp, ix, ssm->d_w32, rc->d_start,
                                                                         rc->d_e32, rc->d_x32, ctx->d_queue, stats);
             }
         } else if (pairs) {
