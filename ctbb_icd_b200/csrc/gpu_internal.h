@@ -7,7 +7,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <algorithm>
 #include <atomic>
 #include <vector>
 
@@ -46,78 +45,59 @@ struct ctbb_ctx {
     int* d_flags = nullptr;  // device-side error flags
 };
 
-// Layout of sinograms on the device (error sinogram, FP64 estimate) and of the
-// matrix's sinogram indices: views fastest but for groups of 2^cb channels x 2^rb
-// detector rows (2 x 2),
-//   ((channel >> cb) * nrb + (row >> rb)) * stride + view, then the channel's and
-//   the row's low bits.
-// What bounds the kernels that read it is not bytes but requests: a voxel meets a
-// few neighbouring channels and two rows per view, and its channels drift slowly
-// from view to view, so in the raw data's order (row fastest) neighbouring entries
-// each lie in another 128-byte line. Here a line holds 8 views of a group and a
-// 32-byte sector two: the 16 entry pairs of a warp's load touch 5.3 lines and 13.3
-// sectors instead of 15.5 and 17 (512 x 512 x 64 benchmark; 6.9 and 10.3 on 2.3 mm
-// voxels; groups of 4 rows of one channel: 5.4 and 13.8, 9.7 and 14.3). A slice's
-// first view still adds a constant (s << shift()) to every index of a column.
-// Channels and rows are padded to whole groups, views to whole lines; padding
-// holds zeros. Where that would not fit a 31-bit index, nothing is grouped.
+// Second layout of a sinogram, for the bulk-staged kernels with many updates in
+// flight (bulk_layout_pays): views fastest but for groups of 2 channels x 2 rows,
+//   (((channel >> 1) * row groups + (row >> 1)) * stride + view) * 4, then the
+//   channel's and the row's low bits.
+// What bounds those launches is not bytes but requests: a voxel meets a few
+// neighbouring channels and two rows per view, and its channels drift slowly from
+// view to view, so in the raw data's order (row fastest) neighbouring entries each
+// lie in another 128-byte line. Here a line holds 8 views of a group and a 32-byte
+// sector two: the 16 entry pairs of a warp's load touch 5.3 lines and 13.3 sectors
+// instead of 15.5 and 17 (512 x 512 x 64 benchmark; 6.9 and 10.3 on 2.3 mm voxels;
+// groups of 4 rows of one channel: 5.4 and 13.8, 9.7 and 14.3). A slice's first view
+// still adds a constant to every index of a column. Channels and rows are padded to
+// whole groups, views to whole lines; padding holds zeros. stride 0: the raw data's
+// order, also where there is one row or channel or the index would not fit 31 bits.
 struct SinoLayout {
-    int rb = 0, cb = 0, nr = 0, nch = 0, nrb = 0, ncb = 0;
+    int nr = 0, nch = 0, nrb = 0, ncb = 0;
     uint32_t stride = 0;  // views, padded
 
-    static SinoLayout make(uint64_t nch, uint64_t nr, uint64_t views) {
+    static SinoLayout raw() { return SinoLayout(); }
+    static SinoLayout grouped(uint64_t nch, uint64_t nr, uint64_t views) {
         SinoLayout l;
+        const uint64_t nrb = (nr + 1) / 2, ncb = (nch + 1) / 2, stride = (views + 7) / 8 * 8;
+        if (nr < 2 || nch < 2 || ncb * nrb * stride * 4 >= 2147483648ull) return l;
         l.nr = (int)nr;
         l.nch = (int)nch;
-        l.rb = nr >= 2 ? 1 : 0;
-        l.cb = nch >= 2 ? 1 : 0;
-        l.nrb = (l.nr + l.rb) >> l.rb;
-        l.ncb = (l.nch + l.cb) >> l.cb;
-        l.stride = (uint32_t)((views + 7) / 8 * 8);
-        if (l.size() >= 2147483648ull) {
-            l.rb = l.cb = 0;
-            l.nrb = l.nr;
-            l.ncb = l.nch;
-            l.stride = (uint32_t)views;
-        }
+        l.nrb = (int)nrb;
+        l.ncb = (int)ncb;
+        l.stride = (uint32_t)stride;
         return l;
     }
-    __host__ __device__ int shift() const { return rb + cb; }
-    uint64_t size() const { return ((uint64_t)ncb * nrb * stride) << (rb + cb); }
+    bool is_raw() const { return stride == 0; }
+    // Elements of a sinogram (grouped layouts).
+    uint64_t size() const { return (uint64_t)ncb * nrb * stride * 4; }
     __host__ __device__ uint32_t at(uint32_t view, uint32_t ch, uint32_t row) const {
-        return ((((ch >> cb) * (uint32_t)nrb + (row >> rb)) * stride + view) << (rb + cb)) |
-               ((ch & (uint32_t)cb) << rb) | (row & (uint32_t)rb);
+        return (((ch >> 1) * (uint32_t)nrb + (row >> 1)) * stride + view) * 4 + (ch & 1) * 2 + (row & 1);
     }
-    // The inverse; rows, channels and views of the padding come out past the end.
-    __host__ __device__ void split(uint32_t a, uint32_t* view, uint32_t* ch, uint32_t* row) const {
-        const uint32_t t = a >> (rb + cb), u = t / stride, c = u / (uint32_t)nrb;
-        *view = t - u * stride;
-        *ch = (c << cb) | ((a >> rb) & (uint32_t)cb);
-        *row = ((u - c * (uint32_t)nrb) << rb) | (a & (uint32_t)rb);
-    }
-    // The raw data's order (row fastest).
-    __host__ __device__ uint32_t linear(uint32_t a) const {
-        uint32_t v, c, r;
-        split(a, &v, &c, &r);
-        return r + (uint32_t)nr * (c + (uint32_t)nch * v);
-    }
-    __host__ __device__ uint32_t from_linear(uint32_t q) const {
+    // Index of the raw data's element q = row + nr * (channel + nch * view).
+    __host__ __device__ uint32_t from_raw(uint32_t q) const {
         const uint32_t t = q / (uint32_t)nr, v = t / (uint32_t)nch;
         return at(v, t - v * (uint32_t)nch, q - t * (uint32_t)nr);
     }
-    // What leads from a row to the next one of the same view and channel: 1 within
-    // a group, row_step() from its last row (low bit set) to the next group.
-    __host__ __device__ uint32_t row_mask() const { return (uint32_t)rb; }
-    __host__ __device__ uint32_t row_step() const { return (stride << (rb + cb)) - (uint32_t)rb; }
-    // Elements of one channel group: an index's quotient by it tells the group.
-    __host__ __device__ uint32_t plane() const { return ((uint32_t)nrb * stride) << (rb + cb); }
-    bool operator==(const SinoLayout& o) const {
-        return rb == o.rb && cb == o.cb && nr == o.nr && nch == o.nch && stride == o.stride;
+    // The same element in a layout of another stride.
+    __host__ __device__ uint32_t restride(uint32_t a, const SinoLayout& to) const {
+        const uint32_t g = a >> 2, line = g / stride;
+        return (line * to.stride + (g - line * stride)) * 4 + (a & 3);
     }
+    // From an odd row to the next row of the same view and channel (from an even one: 1).
+    uint32_t row_step() const { return stride * 4 - 1; }
+    bool operator==(const SinoLayout& o) const { return nr == o.nr && nch == o.nch && stride == o.stride; }
 };
 
 // Stored system matrix: per voxel column c = i + nx*j, entries sorted by
-// q = row + Nrows*(channel + n_channels*view), stored as lay.from_linear(q). colptr[c] is the first entry of
+// q = row + Nrows*(channel + n_channels*view). colptr[c] is the first entry of
 // column c; vptr[c*(nvsm+1) + v] is the offset (relative to colptr[c]) of the
 // first entry of SSM view v, so a view window [v0, v1) is one contiguous run.
 struct ctbb_ssm {
@@ -131,7 +111,6 @@ struct ctbb_ssm {
         return ++n;
     }
     ctbb_geom_c geom{};
-    SinoLayout lay;
     uint64_t ncol = 0, nvsm = 0, nnz = 0, max_col_nnz = 0;
     int64_t* d_colptr = nullptr;  // [ncol + 1]
     uint32_t* d_vptr = nullptr;   // [ncol * (nvsm + 1)]
@@ -144,8 +123,11 @@ struct ctbb_ssm {
     int64_t* d_pcolptr = nullptr;  // [ncol + 1]
     uint32_t* d_pvptr = nullptr;   // [ncol * (nvsm + 1)]
     uint2* d_pairs = nullptr;      // [npairs]
-    uint64_t npairs = 0;       // runs of two consecutive q (reported)
+    uint64_t npairs = 0;
     bool pairs_checked = false;  // build tried (pairs kept only where they pay)
+    bool pairs_pay = false;      // and kept
+    SinoLayout pair_lay;         // of the pairs' indices; entries keep the raw data's order
+    uint64_t pairs_id = 0;       // changes with every build of the pairs
     int weights = 0;
     int ffs = 0;
     double build_ms = 0.0;
@@ -158,16 +140,16 @@ struct ctbb_ssm {
 struct ctbb_recon {
     ctbb_ctx* ctx = nullptr;
     ctbb_geom_c geom{};
-    SinoLayout lay;
     uint64_t nvox = 0, data_size = 0;
-    uint64_t sino_size = 0;  // elements of d_est64 and d_e32 (lay.size())
     std::vector<uint64_t> slice_indices;
     int32_t* d_start = nullptr;  // [nz] first data view of each slice's SSM window
     float* d_raw = nullptr;      // y
     double* d_x64 = nullptr;     // sequential-mode image
     double* d_est64 = nullptr;   // sequential-mode A x (FP64); also FP64 refresh accumulator
     float* d_x32 = nullptr;      // grouped-mode image
-    float* d_e32 = nullptr;      // grouped-mode y - A x; sequential mode: y in the same layout
+    float* d_e32 = nullptr;      // grouped-mode y - A x
+    SinoLayout bulk_lay;         // the second layout of this scan
+    bool e_bulk = false;         // d_e32 is in it (else in the raw data's order)
     int rep = 0;                 // 0: x64/est64 current, 1: x32/e32 current
     // Sum over voxels inside the FOV of in-range matrix entries (cached per matrix).
     uint64_t entries_ssm = 0;
@@ -206,16 +188,16 @@ ctbb_status ensure_partials(ctbb_ctx* ctx, size_t n);
 
 // ssm.cu
 ctbb_status ssm_validate_geometry(const ctbb_geom_c& g);
-ctbb_status ssm_build_pairs(ctbb_ssm* s);
-ctbb_status ssm_relayout(ctbb_ssm* s, const SinoLayout& to);
+// The pair form with its indices in `lay`; no pairs where they do not pay.
+ctbb_status ssm_build_pairs(ctbb_ssm* s, const SinoLayout& lay);
 
 // recon.cu
+// Refuses a matrix of another geometry or context.
+ctbb_status check_pair(const ctbb_recon* rc, const ctbb_ssm* ssm);
+// Grouped mode: the error sinogram in the second layout or in the raw data's order.
+ctbb_status arrange_error(ctbb_recon* rc, bool bulk);
 ctbb_status recon_to_grouped(ctbb_recon* rc, const ctbb_ssm* ssm);
 ctbb_status recon_to_sequential(ctbb_recon* rc, const ctbb_ssm* ssm);
-ctbb_status arranged_raw(ctbb_recon* rc);  // y in the device layout into d_e32
-ctbb_status match_layout(ctbb_recon* rc, const ctbb_ssm* ssm);
-// Refuses a matrix of another geometry or context, then match_layout.
-ctbb_status check_pair(ctbb_recon* rc, const ctbb_ssm* ssm);
 ctbb_status forward_project_f64(ctbb_recon* rc, const ctbb_ssm* ssm, bool from_x32, double* d_out);
 ctbb_status cost_f64(ctbb_recon* rc, const ctbb_ssm* ssm, bool exact, double* out);
 

@@ -60,12 +60,7 @@
 namespace {
 
 struct GParams {
-    int nx, ny, nz, nvsm, readings, penalty;
-    // Sinogram layout (SinoLayout): a slice's first view adds s << view_shift to its
-    // indices; the next detector row is 1 or, where the row_mask bits are set,
-    // row_step further.
-    int view_shift;
-    uint32_t row_mask, row_step;
+    int nx, ny, nz, nch, nr, nvsm, readings, penalty;
     int last_slice[2];  // last slice of each parity
     uint64_t n_items, nvsm1;
     double lambda, delta;
@@ -153,9 +148,10 @@ __device__ __forceinline__ void load_chunk(const int32_t* __restrict__ idx, cons
 }
 
 // Sinogram index of a pair's entry: the pair's own row a, or the next one.
-__device__ __forceinline__ int pair_index(const GParams& P, uint32_t a, int off, int half) {
-    const uint32_t step = (a & P.row_mask) == P.row_mask ? P.row_step : 1u;
-    return (int)a + off + (half ? (int)step : 0);
+template <bool GROUPED>
+__device__ __forceinline__ int pair_index(uint32_t a, int off, int half, uint32_t row_step) {
+    if (GROUPED) return (int)(a + (half ? ((a & 1) ? row_step : 1u) : 0u)) + off;
+    return (int)a + off + half;
 }
 
 // The two FP16 weights of an entry pair ({q, w0 | w1 << 16}).
@@ -463,7 +459,7 @@ __device__ __forceinline__ void process_item(const GParams& P, const uint32_t* _
         const int vs = min(max(start[kl] - s, v0), v1);
         mid = cb + vp[vs];
     }
-    const int off = s * (1 << P.view_shift);
+    const int off = s * P.nch * P.nr;
 
     // beta = sum a e, alpha = sum a^2 (FP32 accumulation per lane) over
     // [mid, en) then [b, mid).
@@ -527,9 +523,10 @@ __global__ void __launch_bounds__(256) icd_grouped_kernel(GParams P, const uint3
 // rows as with single entries (coalesced in the same sectors) while the
 // matrix costs 4 bytes per entry instead of 6. Position p of a lane in row u
 // of a chunk: pair base + 16 u + lane / 2, entry lane & 1.
-template <int U, int STRIDE = 16>
-__device__ __forceinline__ void load_pair_entries(const GParams& P, const uint2* __restrict__ pairs, int64_t m, int64_t en, int off,
-                                                  int half, uint64_t pol, int* q, float* wt) {
+// GROUPED: the pairs' indices are in the second sinogram layout.
+template <int U, int STRIDE = 16, bool GROUPED = false>
+__device__ __forceinline__ void load_pair_entries(const uint2* __restrict__ pairs, int64_t m, int64_t en, int off,
+                                                  int half, uint64_t pol, int* q, float* wt, uint32_t row_step = 1) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         const int64_t mu = m + (int64_t)STRIDE * u;
@@ -541,7 +538,7 @@ __device__ __forceinline__ void load_pair_entries(const GParams& P, const uint2*
                          : "=r"(a), "=r"(bb)
                          : "l"(pairs + mu), "l"(pol));
             if (!half || (bb >> 16)) {
-                q[u] = pair_index(P, a, off, half);
+                q[u] = pair_index<GROUPED>(a, off, half, row_step);
                 wt[u] = half ? half_hi(bb) : half_lo(bb);
             }
         }
@@ -551,7 +548,7 @@ __device__ __forceinline__ void load_pair_entries(const GParams& P, const uint2*
 // Pair positions p, p + STRIDE, ... of an item's sweep: pair p + hi for
 // p < n1, else p + lo; -1 / 0 past n (the sweep's length).
 template <int U, int STRIDE>
-__device__ __forceinline__ void load_seq_pairs(const GParams& P, const uint2* __restrict__ pairs, int p0, int n, int n1, int64_t hi,
+__device__ __forceinline__ void load_seq_pairs(const uint2* __restrict__ pairs, int p0, int n, int n1, int64_t hi,
                                                int64_t lo, int off, int half, uint64_t pol, int* q, float* wt) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -565,7 +562,7 @@ __device__ __forceinline__ void load_seq_pairs(const GParams& P, const uint2* __
                          : "=r"(a), "=r"(bb)
                          : "l"(pairs + m), "l"(pol));
             if (!half || (bb >> 16)) {
-                q[u] = pair_index(P, a, off, half);
+                q[u] = (int)a + off + half;
                 wt[u] = half ? half_hi(bb) : half_lo(bb);
             }
         }
@@ -573,20 +570,20 @@ __device__ __forceinline__ void load_seq_pairs(const GParams& P, const uint2* __
 }
 
 template <int U>
-__device__ __forceinline__ void gather_pairs(const GParams& P, const uint2* __restrict__ pairs, const float* e, int64_t b, int64_t en,
+__device__ __forceinline__ void gather_pairs(const uint2* __restrict__ pairs, const float* e, int64_t b, int64_t en,
                                              int off, int lane, uint64_t pol, float& acc_b, float& acc_a) {
     if (b >= en) return;
     const int half = lane & 1, j = lane >> 1;
     int qa[U];
     float wa[U];
-    load_pair_entries<U>(P, pairs, b + j, en, off, half, pol, qa, wa);
+    load_pair_entries<U>(pairs, b + j, en, off, half, pol, qa, wa);
     for (int64_t base = b; base < en; base += 16 * U) {
         float ev[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) ev[u] = qa[u] >= 0 ? __ldcg(e + qa[u]) : 0.f;
         int qb[U];
         float wb[U];
-        load_pair_entries<U>(P, pairs, base + 16 * U + j, en, off, half, pol, qb, wb);
+        load_pair_entries<U>(pairs, base + 16 * U + j, en, off, half, pol, qb, wb);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             acc_b = fmaf(wa[u], ev[u], acc_b);
@@ -598,7 +595,7 @@ __device__ __forceinline__ void gather_pairs(const GParams& P, const uint2* __re
 }
 
 template <int U>
-__device__ __forceinline__ void scatter_pairs(const GParams& P, const uint2* __restrict__ pairs, float* e, int64_t b, int64_t en,
+__device__ __forceinline__ void scatter_pairs(const uint2* __restrict__ pairs, float* e, int64_t b, int64_t en,
                                               int off, int lane, uint64_t pol, float du) {
     if (b >= en) return;
     const int half = lane & 1, j = lane >> 1;
@@ -606,7 +603,7 @@ __device__ __forceinline__ void scatter_pairs(const GParams& P, const uint2* __r
     for (int64_t c = nchunk - 1; c >= 0; --c) {
         int qs[U];
         float ws[U];
-        load_pair_entries<U>(P, pairs, b + c * (16 * U) + j, en, off, half, pol, qs, ws);
+        load_pair_entries<U>(pairs, b + c * (16 * U) + j, en, off, half, pol, qs, ws);
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (qs[u] >= 0) atomicAdd(e + qs[u], -du * ws[u]);
@@ -645,11 +642,11 @@ __global__ void __launch_bounds__(256) icd_grouped_pairs_kernel(
             mid = cb + vp[min(max(start[kl] - s, v0), v1)];
             n_entries = (int64_t)vptr[col * P.nvsm1 + v1] - (int64_t)vptr[col * P.nvsm1 + v0];
         }
-        const int off = s * (1 << P.view_shift);
+        const int off = s * P.nch * P.nr;
         float acc_b = 0.f, acc_a = 0.f;
         const uint64_t keep = l2_keep();
-        gather_pairs<U>(P, pairs, e, mid, en, off, lane, keep, acc_b, acc_a);
-        gather_pairs<U>(P, pairs, e, b, mid, off, lane, keep, acc_b, acc_a);
+        gather_pairs<U>(pairs, e, mid, en, off, lane, keep, acc_b, acc_a);
+        gather_pairs<U>(pairs, e, b, mid, off, lane, keep, acc_b, acc_a);
         const double beta = (double)warp_sum(acc_b);
         const double alpha = (double)warp_sum(acc_a);
         const double xq = (double)__ldcg(x + q);
@@ -659,8 +656,8 @@ __global__ void __launch_bounds__(256) icd_grouped_pairs_kernel(
         const float du = (float)upd;
         if (du != 0.f) {
             const uint64_t drop = l2_drop();
-            scatter_pairs<U>(P, pairs, e, b, mid, off, lane, drop, du);
-            scatter_pairs<U>(P, pairs, e, mid, en, off, lane, drop, du);
+            scatter_pairs<U>(pairs, e, b, mid, off, lane, drop, du);
+            scatter_pairs<U>(pairs, e, mid, en, off, lane, drop, du);
             n_ent += (unsigned long long)n_entries;
             ++n_upd;
         }
@@ -734,7 +731,7 @@ __global__ void __launch_bounds__(32 * WPV, 16 / WPV) icd_cta_pairs_kernel(
             mid = P.stack_align ? cb + vp[stack_start_view(P, start, k, s, v0, v1)] : b;
             if (tid == 0) n_entries = (int64_t)vptr[col * P.nvsm1 + v1] - (int64_t)vptr[col * P.nvsm1 + v0];
         }
-        const int off = s * (1 << P.view_shift);
+        const int off = s * P.nch * P.nr;
         // Sweep position p (pairs) -> pair p + hi for p < n1 ([mid, en)), else
         // p + lo ([b, mid)).
         const int n = (int)(en - b), n1 = (int)(en - mid);
@@ -754,7 +751,7 @@ __global__ void __launch_bounds__(32 * WPV, 16 / WPV) icd_cta_pairs_kernel(
                              : "=r"(a), "=r"(bb)
                              : "l"(pairs + m), "l"(pol_m));
                 if (!half || (bb >> 16)) {
-                    qr[r] = pair_index(P, a, off, half);
+                    qr[r] = (int)a + off + half;
                     wr[r] = half ? half_hi(bb) : half_lo(bb);
                 }
             }
@@ -769,7 +766,7 @@ __global__ void __launch_bounds__(32 * WPV, 16 / WPV) icd_cta_pairs_kernel(
         for (int base = (int)CAP; base < n; base += NP * kU) {
             int qo[kU];
             float wo[kU];
-            load_seq_pairs<kU, NP>(P, pairs, base + j, n, n1, hi, lo, off, half, pol_m, qo, wo);
+            load_seq_pairs<kU, NP>(pairs, base + j, n, n1, hi, lo, off, half, pol_m, qo, wo);
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
                 const float ev = qo[u] >= 0 ? ld_e(e + qo[u], pol_e) : 0.f;
@@ -808,7 +805,7 @@ __global__ void __launch_bounds__(32 * WPV, 16 / WPV) icd_cta_pairs_kernel(
             for (int base = (int)CAP; base < n; base += NP * kU) {
                 int qo[kU];
                 float wo[kU];
-                load_seq_pairs<kU, NP>(P, pairs, base + j, n, n1, hi, lo, off, half, pol_m, qo, wo);
+                load_seq_pairs<kU, NP>(pairs, base + j, n, n1, hi, lo, off, half, pol_m, qo, wo);
 #pragma unroll
                 for (int u = 0; u < kU; ++u)
                     if (qo[u] >= 0) atomicAdd(e + qo[u], -du * wo[u]);
@@ -893,6 +890,7 @@ __device__ __forceinline__ void bulk_g2s_hint(uint32_t dst, const void* src, uin
 // b0 = b rounded down and e1 rounded up to even (16-byte boundaries; the pair
 // array has two pairs of padding past its end); the item's first pair sits at
 // stage position d = b - b0.
+template <bool GROUPED>
 __device__ __forceinline__ void bulk_issue(const GParams& P, const uint32_t* __restrict__ order,
                                            const int64_t* __restrict__ pcolptr, const uint32_t* __restrict__ pvptr,
                                            const uint2* __restrict__ pairs, const uint32_t* __restrict__ vptr,
@@ -925,7 +923,7 @@ __device__ __forceinline__ void bulk_issue(const GParams& P, const uint32_t* __r
     it->en = en;
     it->q = (int64_t)col + (int64_t)ncol * k;
     it->n_entries = ne;
-    it->off = s * (1 << P.view_shift);
+    it->off = GROUPED ? s * 4 : s * P.nch * P.nr;
     it->d = (int)(b - b0);
     it->ns = ns;
     it->valid = 1;
@@ -945,12 +943,13 @@ __device__ __forceinline__ void bulk_issue(const GParams& P, const uint32_t* __r
     }
 }
 
-template <int STAGES>
+// GROUPED: e and the pairs' indices are in the second sinogram layout.
+template <int STAGES, bool GROUPED>
 __global__ void __launch_bounds__(kBulkThreads, STAGES == 1 ? 4 : 3) icd_bulk_kernel(
     GParams P, const uint32_t* __restrict__ order, const int64_t* __restrict__ pcolptr,
     const uint32_t* __restrict__ pvptr, const uint2* __restrict__ pairs, const uint32_t* __restrict__ vptr,
     const int32_t* __restrict__ start, float* e, float* x, unsigned long long* queue, unsigned long long* stats,
-    unsigned long long* err) {
+    unsigned long long* err, uint32_t row_step) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ float s_red[2 * (kBulkThreads / 32) + 1];
     constexpr int NW = kBulkThreads / 32;
@@ -966,7 +965,7 @@ __global__ void __launch_bounds__(kBulkThreads, STAGES == 1 ? 4 : 3) icd_bulk_ke
         for (int s = 0; s < STAGES; ++s) bulk_mbar_init(bar(s), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         for (int s = 0; s < STAGES; ++s)
-            bulk_issue(P, order, pcolptr, pvptr, pairs, vptr, start, queue, &items[s], stage_addr(s), bar(s));
+            bulk_issue<GROUPED>(P, order, pcolptr, pvptr, pairs, vptr, start, queue, &items[s], stage_addr(s), bar(s));
     }
     uint32_t parity = 0;  // bit s: phase of stage s's barrier to wait for
     int cur = 0;
@@ -998,7 +997,7 @@ __global__ void __launch_bounds__(kBulkThreads, STAGES == 1 ? 4 : 3) icd_bulk_ke
             float v = 0.f;
             if (p < it.ns) {
                 const uint2 pr = stp[p];
-                if (!half || (pr.y >> 16)) v = __ldcg(e + pair_index(P, pr.x, it.off, half));
+                if (!half || (pr.y >> 16)) v = __ldcg(e + pair_index<GROUPED>(pr.x, it.off, half, row_step));
             }
             ev[i] = v;
         }
@@ -1016,7 +1015,8 @@ __global__ void __launch_bounds__(kBulkThreads, STAGES == 1 ? 4 : 3) icd_bulk_ke
         for (int b2 = it.ns; b2 < n; b2 += kBulkNP * kU) {
             int qo[kU];
             float wo[kU];
-            load_pair_entries<kU, kBulkNP>(P, pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
+            load_pair_entries<kU, kBulkNP, GROUPED>(pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo,
+                                                    row_step);
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
                 const float evu = qo[u] >= 0 ? __ldcg(e + qo[u]) : 0.f;
@@ -1056,13 +1056,15 @@ __global__ void __launch_bounds__(kBulkThreads, STAGES == 1 ? 4 : 3) icd_bulk_ke
                 if (p < it.ns) {
                     const uint2 pr = stp[p];
                     if (!half || (pr.y >> 16))
-                        atomicAdd(e + pair_index(P, pr.x, it.off, half), -du * (half ? half_hi(pr.y) : half_lo(pr.y)));
+                        atomicAdd(e + pair_index<GROUPED>(pr.x, it.off, half, row_step),
+                                  -du * (half ? half_hi(pr.y) : half_lo(pr.y)));
                 }
             }
             for (int b2 = it.ns; b2 < n; b2 += kBulkNP * kU) {
                 int qo[kU];
                 float wo[kU];
-                load_pair_entries<kU, kBulkNP>(P, pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
+                load_pair_entries<kU, kBulkNP, GROUPED>(pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo,
+                                                    row_step);
 #pragma unroll
                 for (int u = 0; u < kU; ++u)
                     if (qo[u] >= 0) atomicAdd(e + qo[u], -du * wo[u]);
@@ -1072,7 +1074,8 @@ __global__ void __launch_bounds__(kBulkThreads, STAGES == 1 ? 4 : 3) icd_bulk_ke
         }
         __syncthreads();  // the stage, the item record and s_red are free
         if (tid == 0)
-            bulk_issue(P, order, pcolptr, pvptr, pairs, vptr, start, queue, &items[cur], stage_addr(cur), bar(cur));
+            bulk_issue<GROUPED>(P, order, pcolptr, pvptr, pairs, vptr, start, queue, &items[cur], stage_addr(cur),
+                                bar(cur));
         cur = cur + 1 == STAGES ? 0 : cur + 1;
     }
     if (failed) {
@@ -1102,6 +1105,7 @@ __global__ void __launch_bounds__(kBulkThreads, STAGES == 1 ? 4 : 3) icd_bulk_ke
 // re-reading the pairs from global memory, measured slower: the re-read
 // column mostly missed L2 and DRAM bytes per entry rose by 39 %.)
 // ---------------------------------------------------------------------------
+template <bool GROUPED>
 __device__ __forceinline__ void bulk_claim(const GParams& P, const uint32_t* __restrict__ order,
                                            const int64_t* __restrict__ pcolptr, const uint32_t* __restrict__ pvptr,
                                            const uint32_t* __restrict__ vptr, const int32_t* __restrict__ start,
@@ -1130,7 +1134,7 @@ __device__ __forceinline__ void bulk_claim(const GParams& P, const uint32_t* __r
     it->en = en;
     it->q = (int64_t)col + (int64_t)ncol * k;
     it->n_entries = ne;
-    it->off = s * (1 << P.view_shift);
+    it->off = GROUPED ? s * 4 : s * P.nch * P.nr;
     it->d = (int)(b - (b & ~(int64_t)1));
     it->ns = ns;
     it->valid = 1;
@@ -1152,11 +1156,12 @@ __device__ __forceinline__ void bulk_copy(const uint2* __restrict__ pairs, const
     for (uint32_t o = 0; o < bytes; o += kBulkChunk) bulk_g2s(dst + o, src + o, min(kBulkChunk, bytes - o), bar);
 }
 
+template <bool GROUPED>
 __global__ void __launch_bounds__(kBulkThreads, 4) icd_bulk_pipe_kernel(
     GParams P, const uint32_t* __restrict__ order, const int64_t* __restrict__ pcolptr,
     const uint32_t* __restrict__ pvptr, const uint2* __restrict__ pairs, const uint32_t* __restrict__ vptr,
     const int32_t* __restrict__ start, float* e, float* x, unsigned long long* queue, unsigned long long* stats,
-    unsigned long long* err) {
+    unsigned long long* err, uint32_t row_step) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ float s_red[2 * (kBulkThreads / 32) + 1];
     constexpr int NW = kBulkThreads / 32;
@@ -1172,7 +1177,7 @@ __global__ void __launch_bounds__(kBulkThreads, 4) icd_bulk_pipe_kernel(
     if (tid == 0) {
         bulk_mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        bulk_claim(P, order, pcolptr, pvptr, vptr, start, queue, &ring[0]);
+        bulk_claim<GROUPED>(P, order, pcolptr, pvptr, vptr, start, queue, &ring[0]);
         if (ring[0].valid) bulk_copy(pairs, ring[0], stage, bar);
     }
     uint32_t parity = 0;
@@ -1204,7 +1209,7 @@ __global__ void __launch_bounds__(kBulkThreads, 4) icd_bulk_pipe_kernel(
             float v = 0.f;
             if (p < it.ns) {
                 const uint2 pr = stp[p];
-                if (!half || (pr.y >> 16)) v = __ldcg(e + pair_index(P, pr.x, it.off, half));
+                if (!half || (pr.y >> 16)) v = __ldcg(e + pair_index<GROUPED>(pr.x, it.off, half, row_step));
             }
             ev[i] = v;
         }
@@ -1222,7 +1227,8 @@ __global__ void __launch_bounds__(kBulkThreads, 4) icd_bulk_pipe_kernel(
         for (int b2 = it.ns; b2 < n; b2 += kBulkNP * kU) {
             int qo[kU];
             float wo[kU];
-            load_pair_entries<kU, kBulkNP>(P, pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
+            load_pair_entries<kU, kBulkNP, GROUPED>(pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo,
+                                                    row_step);
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
                 const float evu = qo[u] >= 0 ? __ldcg(e + qo[u]) : 0.f;
@@ -1255,7 +1261,7 @@ __global__ void __launch_bounds__(kBulkThreads, 4) icd_bulk_pipe_kernel(
         } else if (tid == 32) {
             // The next item, claimed while warp 0 solves (the slot held the
             // item finished last round, no longer read).
-            bulk_claim(P, order, pcolptr, pvptr, vptr, start, queue, &ring[nxt]);
+            bulk_claim<GROUPED>(P, order, pcolptr, pvptr, vptr, start, queue, &ring[nxt]);
         }
         __syncthreads();
         const float du = s_red[2 * NW];
@@ -1266,13 +1272,15 @@ __global__ void __launch_bounds__(kBulkThreads, 4) icd_bulk_pipe_kernel(
                 if (p < it.ns) {
                     const uint2 pr = stp[p];
                     if (!half || (pr.y >> 16))
-                        atomicAdd(e + pair_index(P, pr.x, it.off, half), -du * (half ? half_hi(pr.y) : half_lo(pr.y)));
+                        atomicAdd(e + pair_index<GROUPED>(pr.x, it.off, half, row_step),
+                                  -du * (half ? half_hi(pr.y) : half_lo(pr.y)));
                 }
             }
             for (int b2 = it.ns; b2 < n; b2 += kBulkNP * kU) {
                 int qo[kU];
                 float wo[kU];
-                load_pair_entries<kU, kBulkNP>(P, pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo);
+                load_pair_entries<kU, kBulkNP, GROUPED>(pairs, it.b + b2 + j, it.en, it.off, half, pol, qo, wo,
+                                                    row_step);
 #pragma unroll
                 for (int u = 0; u < kU; ++u)
                     if (qo[u] >= 0) atomicAdd(e + qo[u], -du * wo[u]);
@@ -1347,7 +1355,7 @@ __global__ void __launch_bounds__(32 * kStack, U == 8 ? 2 : 1) icd_lockstep_kern
                     hi = cb + mid;
                     lo = cb + b - n1;
                 }
-                off = s * (1 << P.view_shift);
+                off = s * P.nch * P.nr;
             }
             const int chunks = (n + 32 * U - 1) / (32 * U);
             if (lane == 0) s_chunks[wid] = chunks;
@@ -1455,7 +1463,7 @@ __device__ __forceinline__ void staged_item(const GParams& P, const uint32_t* __
         const int vs = min(max(start[kl] - s, v0), v1);
         mid = cb + vp[vs];
     }
-    const int off = s * (1 << P.view_shift);
+    const int off = s * P.nch * P.nr;
     const int64_t n1 = en - mid, n = en - b;
 
     float acc_b = 0.f, acc_a = 0.f;
@@ -1566,7 +1574,7 @@ __global__ void __launch_bounds__(32 * WPV, 16 / WPV) icd_cta_kernel(GParams P, 
             en = cb + vp[v1];
             mid = P.stack_align ? cb + vp[stack_start_view(P, start, k, s, v0, v1)] : b;
         }
-        const int off = s * (1 << P.view_shift);
+        const int off = s * P.nch * P.nr;
         // Sweep position p -> entry p + hi for p < n1 ([mid, en)), else p + lo
         // ([b, mid)).
         const int n = (int)(en - b), n1 = (int)(en - mid);
@@ -1820,9 +1828,8 @@ GParams make_params(const ctbb_recon* rc, const ctbb_ssm* ssm, const ctbb_icd_op
     P.nx = (int)g.num_voxels_x;
     P.ny = (int)g.num_voxels_y;
     P.nz = (int)g.num_voxels_z;
-    P.view_shift = rc->lay.shift();
-    P.row_mask = rc->lay.row_mask();
-    P.row_step = rc->lay.row_step();
+    P.nch = (int)g.n_channels;
+    P.nr = (int)g.Nrows_projection;
     P.nvsm = (int)ssm->nvsm;
     P.nvsm1 = ssm->nvsm + 1;
     P.readings = (int)g.Readings;
@@ -2080,6 +2087,7 @@ ctbb_status launch_staged(const GParams& P, const uint32_t* order, const ctbb_ss
 struct GraphKey {
     GParams P;
     uint64_t ssm;  // the matrix (its id, not its address)
+    uint64_t pairs_id;
     const void* order;
     const void* stacks;
     const void* w;
@@ -2090,6 +2098,18 @@ struct GraphKey {
     int stage, pairs, wpv, epl, h;
 };
 
+
+// The one-stage bulk kernels take the second sinogram layout with more than three
+// updates an SM in flight, where L2 and DRAM sectors bound them (one iteration at
+// four an SM: 201 x 201 x 37 61.8 -> 37.4 ms, 137 x 137 x 29 at 2 mm 97 -> 84; at two
+// 71.9 -> 63 and 158 -> 141). Below, latency bounds them, and a layout that shortens
+// the gather more than the reductions changes which updates an update sees: on
+// voxels of many channels the image after one iteration lay 1.4-2.9 times the
+// raw order's run-to-run distance away at one to three updates an SM, and 0.7-1.3
+// times at four.
+bool bulk_layout_pays(const ctbb_recon* rc, int stage, uint64_t in_flight) {
+    return (stage == 4 || stage == 6) && in_flight > 3 * (uint64_t)rc->ctx->sm_count && !rc->bulk_lay.is_raw();
+}
 
 // Build (or reuse) the full visiting order for tile edge P_lat.
 ctbb_status build_order(ctbb_recon* rc, int P_lat) {
@@ -2190,12 +2210,16 @@ ctbb_status launch_icd_grouped(ctbb_recon* rc, const ctbb_ssm* ssm, const ctbb_i
     // Entry pairs for the CTA-per-update kernels with FP16 weights (built
     // here, outside any stream capture, on first use).
     const bool want_pairs = h && (stage >= 4 || (o.entry_pairs == 0 && (wpv > 1 || stage == 0)));
-    if (want_pairs) CTBB_TRY(ssm_build_pairs(const_cast<ctbb_ssm*>(ssm)));
+    // (the claim-ahead kernel holds two items per CTA, so half the order's bound in CTAs)
+    const bool bulk = bulk_layout_pays(rc, stage, stage == 6 ? std::min(in_flight, order_bound / 2) : in_flight);
+    if (want_pairs) CTBB_TRY(ssm_build_pairs(const_cast<ctbb_ssm*>(ssm), bulk ? rc->bulk_lay : SinoLayout::raw()));
     const bool pairs = want_pairs && ssm->d_pairs;
     if (stage >= 4 && !pairs)
         return fail(CTBB_ERR_INVALID_ARG,
                     "stage_column 4-6 reads entry pairs: needs FP16 weights and a matrix whose detector-row runs "
                     "pair up (no z flying focal spot)");
+    CTBB_TRY(arrange_error(rc, bulk));
+    const uint32_t row_step = bulk ? rc->bulk_lay.row_step() : 1;
     const int64_t* cp = ssm->d_colptr;
     const uint32_t* vp = ssm->d_vptr;
     const int32_t* ix = ssm->d_idx;
@@ -2208,40 +2232,32 @@ ctbb_status launch_icd_grouped(ctbb_recon* rc, const ctbb_ssm* ssm, const ctbb_i
             // Claim-ahead bulk-staged kernel: one stage, two claimed items
             // per CTA, so half the order's bound in CTAs.
             const size_t smem = bulk_smem_bytes(1);
+            const auto kernel = bulk ? icd_bulk_pipe_kernel<true> : icd_bulk_pipe_kernel<false>;
             if (prepare) {
-                CTBB_CUDA(cudaFuncSetAttribute(icd_bulk_pipe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem));
+                CTBB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 return CTBB_OK;
             }
             const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(in_flight, order_bound / 2));
-            icd_bulk_pipe_kernel<<<blocks, kBulkThreads, smem, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr,
-                                                                     ssm->d_pairs, vp, rc->d_start, rc->d_e32,
-                                                                     rc->d_x32, ctx->d_queue, stats, stats + 2);
+            kernel<<<blocks, kBulkThreads, smem, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr, ssm->d_pairs, vp,
+                                                      rc->d_start, rc->d_e32, rc->d_x32, ctx->d_queue, stats,
+                                                      stats + 2, row_step);
             CTBB_CUDA(cudaGetLastError());
             return CTBB_OK;
         }
         if (stage >= 4) {
             // One update per CTA of 8 warps; 4: one pair stage, 5: two.
-            const int stages = stage == 4 ? 1 : 2;
-            const size_t smem = bulk_smem_bytes(stages);
+            const size_t smem = bulk_smem_bytes(stage == 4 ? 1 : 2);
+            const auto kernel = stage == 5 ? icd_bulk_kernel<2, false>
+                                : bulk     ? icd_bulk_kernel<1, true>
+                                           : icd_bulk_kernel<1, false>;
             if (prepare) {
-                if (stages == 1)
-                    CTBB_CUDA(cudaFuncSetAttribute(icd_bulk_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)smem));
-                else
-                    CTBB_CUDA(cudaFuncSetAttribute(icd_bulk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)smem));
+                CTBB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 return CTBB_OK;
             }
             const int blocks = (int)std::max<uint64_t>(1, in_flight);
-            if (stages == 1)
-                icd_bulk_kernel<1><<<blocks, kBulkThreads, smem, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr,
-                                                                      ssm->d_pairs, vp, rc->d_start, rc->d_e32,
-                                                                      rc->d_x32, ctx->d_queue, stats, stats + 2);
-            else
-                icd_bulk_kernel<2><<<blocks, kBulkThreads, smem, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr,
-                                                                      ssm->d_pairs, vp, rc->d_start, rc->d_e32,
-                                                                      rc->d_x32, ctx->d_queue, stats, stats + 2);
+            kernel<<<blocks, kBulkThreads, smem, s>>>(P, order, ssm->d_pcolptr, ssm->d_pvptr, ssm->d_pairs, vp,
+                                                      rc->d_start, rc->d_e32, rc->d_x32, ctx->d_queue, stats,
+                                                      stats + 2, row_step);
             CTBB_CUDA(cudaGetLastError());
             return CTBB_OK;
         }
@@ -2366,6 +2382,7 @@ ctbb_status launch_icd_grouped(ctbb_recon* rc, const ctbb_ssm* ssm, const ctbb_i
     key.wpv = wpv;
     key.epl = epl;
     key.h = h;
+    if (pairs) key.pairs_id = ssm->pairs_id;  // and their layout
     const bool have = rc->icd_graph && rc->icd_graph_key.size() == sizeof(key) &&
                       memcmp(rc->icd_graph_key.data(), &key, sizeof(key)) == 0;
     if (!have) {
@@ -2599,20 +2616,13 @@ extern "C" ctbb_status ctbb_gpu_batch_iterate(ctbb_batch* b, const ctbb_icd_opts
                     : std::max(4, std::min(b->ctx->sm_count * 32, (int)(0.4 * n_sum / (3.2 * nx_max))));
     bool orders_changed = b->d_merged == nullptr || b->merged_T.size() != b->recons.size();
     std::vector<int> T(b->recons.size());
-    // Scans that share a matrix settle on one layout: a first pass may move the
-    // matrix to a longer scan's, the second moves the shorter scans to it.
-    for (int pass = 0; pass < 2; ++pass)
-        for (size_t i = 0; i < b->recons.size(); ++i) {
-            const bool moved = !(b->recons[i]->lay == b->ssms[i]->lay);
-            CTBB_TRY(match_layout(b->recons[i], b->ssms[i]));
-            if (moved) drop_graph(b);
-        }
     for (size_t i = 0; i < b->recons.size(); ++i) {
         ctbb_recon* rc = b->recons[i];
         const ctbb_ssm* s = b->ssms[i];
         if ((wsel == CTBB_SSM_FP16 && !s->d_w16) || (wsel == CTBB_SSM_FP32 && !s->d_w32))
             return fail(CTBB_ERR_INVALID_ARG, "scan %zu: matrix does not hold the requested weights", i);
         CTBB_TRY(recon_to_grouped(rc, s));
+        CTBB_TRY(arrange_error(rc, false));
         ctbb_icd_opts oi = o;
         oi.warps_per_voxel = 1;
         oi.warps_in_flight = std::max(1, (int)((double)warps * (double)rc->nvox / n_sum));

@@ -27,8 +27,7 @@
 namespace {
 
 struct SeqParams {
-    int nx, ny, nz, nvsm, readings, penalty;
-    SinoLayout lay;
+    int nx, ny, nz, nch, nr, nvsm, readings, penalty;
     uint64_t nvsm1;
     double cvx, cvy, vx, vy, fov_limit, lambda, delta;
 };
@@ -175,33 +174,34 @@ __global__ void __launch_bounds__(32 * kSeqWarps) icd_seq_kernel(
         }
         return v;
     };
-    // This warp's entries [b, e) of a voxel's in-range column, and the slice's first data view.
-    auto range = [&](const SeqVoxel& v, int64_t& b, int64_t& e, int& s) {
+    // This warp's entries [b, e) of a voxel's in-range column, and the sinogram offset.
+    auto range = [&](const SeqVoxel& v, int64_t& b, int64_t& e, int& off) {
         b = e = 0;
-        s = 0;
+        off = 0;
         if (v.j >= P.ny) return;
-        s = __ldg(start + v.k);
+        const int s = __ldg(start + v.k);
         const int v0 = max(0, -s), v1 = min(P.nvsm, P.readings - s);
         if (v1 <= v0) return;
         const int first = (s + v0) / vb;
         const int g = first + (self - first % nwarps + nwarps) % nwarps;
         const int va = max(v0, g * vb - s), ve = min(v1, (g + 1) * vb - s);
+        off = s * P.nch * P.nr;
         if (va >= ve) return;
         const uint64_t col = (uint64_t)v.i + nxs * v.j;
         const int64_t cb = __ldg(colptr + col);
         b = cb + __ldg(vptr + col * P.nvsm1 + va);
         e = cb + __ldg(vptr + col * P.nvsm1 + ve);
     };
-    // The first kSeqR entries of each lane: sinogram index (-1: none) and weight.
-    auto fetch = [&](int64_t b, int64_t e, int s, int* qi, float* wi) {
-        const uint32_t off = (uint32_t)((int64_t)s << P.lay.shift());  // modulo 2^32: the sum is in range
+    int qi[kSeqR];
+    float wi[kSeqR];
+    auto fetch = [&](int64_t b, int64_t e, int off) {
 #pragma unroll
         for (int r = 0; r < kSeqR; ++r) {
             const int64_t m = b + lane + 32 * r;
             qi[r] = -1;
             wi[r] = 0.f;
             if (m < e) {
-                qi[r] = (int)((uint32_t)__ldg(idx + m) + off);
+                qi[r] = __ldg(idx + m) + off;
                 wi[r] = __ldg(w + m);
             }
         }
@@ -211,12 +211,10 @@ __global__ void __launch_bounds__(32 * kSeqWarps) icd_seq_kernel(
     settle(cur);
     SeqVoxel nx1 = next(cur);
     int64_t b, e, b1, e1;
-    int s0, s1;
-    int qi[kSeqR];
-    float wi[kSeqR];
-    range(cur, b, e, s0);
-    fetch(b, e, s0, qi, wi);
-    range(nx1, b1, e1, s1);
+    int off, off1;
+    range(cur, b, e, off);
+    fetch(b, e, off);
+    range(nx1, b1, e1, off1);
     cluster_arrive();  // every CTA runs before another writes to it
     cluster_wait();
     int par = 0;
@@ -247,10 +245,9 @@ __global__ void __launch_bounds__(32 * kSeqWarps) icd_seq_kernel(
             alpha += (double)ww;
             beta += (double)wi[r] * ((double)rv[r] - ev[r]);
         }
-        const uint32_t off = (uint32_t)((int64_t)s0 << P.lay.shift());
         for (int64_t m = b + 32 * kSeqR + lane; m < e; m += 32) {
             const float wm = __ldg(w + m);
-            const uint32_t index = (uint32_t)__ldg(idx + m) + off;
+            const int index = __ldg(idx + m) + off;
             const float ww = wm * wm;
             alpha += (double)ww;
             beta += (double)wm * ((double)__ldg(raw + index) - est[index]);
@@ -275,11 +272,20 @@ __global__ void __launch_bounds__(32 * kSeqWarps) icd_seq_kernel(
         // While the sums travel: where the voxel after next keeps its entries.
         const SeqVoxel nx2 = next(nx1);
         int64_t b2, e2;
-        int s2;
-        range(nx2, b2, e2, s2);
+        int off2;
+        range(nx2, b2, e2, off2);
         int qn[kSeqR];
         float wn[kSeqR];
-        fetch(b1, e1, s1, qn, wn);
+#pragma unroll
+        for (int r = 0; r < kSeqR; ++r) {
+            const int64_t m = b1 + lane + 32 * r;
+            qn[r] = -1;
+            wn[r] = 0.f;
+            if (m < e1) {
+                qn[r] = __ldg(idx + m) + off1;
+                wn[r] = __ldg(w + m);
+            }
+        }
         cluster_wait();
         if (wid == 0) {
             double2 t = lane < cluster ? s_cta[par][lane] : make_double2(0.0, 0.0);
@@ -300,7 +306,7 @@ __global__ void __launch_bounds__(32 * kSeqWarps) icd_seq_kernel(
         for (int r = 0; r < kSeqR; ++r)
             if (qi[r] >= 0) est[qi[r]] = ev[r] + upd * (double)wi[r];
         for (int64_t m = b + 32 * kSeqR + lane; m < e; m += 32) {
-            const uint32_t index = (uint32_t)__ldg(idx + m) + off;
+            const int index = __ldg(idx + m) + off;
             est[index] += upd * (double)__ldg(w + m);
         }
         __syncwarp();
@@ -308,10 +314,10 @@ __global__ void __launch_bounds__(32 * kSeqWarps) icd_seq_kernel(
         nx1 = nx2;
         b = b1;
         e = e1;
-        s0 = s1;
+        off = off1;
         b1 = b2;
         e1 = e2;
-        s1 = s2;
+        off1 = off2;
 #pragma unroll
         for (int r = 0; r < kSeqR; ++r) {
             qi[r] = qn[r];
@@ -356,7 +362,8 @@ ctbb_status launch_icd_sequential(ctbb_recon* rc, const ctbb_ssm* ssm, int n_ite
     P.nx = (int)g.num_voxels_x;
     P.ny = (int)g.num_voxels_y;
     P.nz = (int)g.num_voxels_z;
-    P.lay = rc->lay;
+    P.nch = (int)g.n_channels;
+    P.nr = (int)g.Nrows_projection;
     P.nvsm = (int)ssm->nvsm;
     P.nvsm1 = ssm->nvsm + 1;
     P.readings = (int)g.Readings;
@@ -373,7 +380,6 @@ ctbb_status launch_icd_sequential(ctbb_recon* rc, const ctbb_ssm* ssm, int n_ite
     CTBB_CUDA(cudaEventCreate(&e0));
     CTBB_CUDA(cudaEventCreate(&e1));
     CTBB_CUDA(cudaEventRecord(e0, st));
-    CTBB_TRY(arranged_raw(rc));  // y beside the estimate, in the estimate's layout
     int cluster = 1;
     CTBB_TRY(seq_cluster(&cluster));
     // Views per block: a window of nvsm views touches at most (warps) blocks.
@@ -392,7 +398,7 @@ ctbb_status launch_icd_sequential(ctbb_recon* rc, const ctbb_ssm* ssm, int n_ite
     for (int it = 0; it < n_iter; ++it)
         CTBB_CUDA(cudaLaunchKernelEx(&cfg, icd_seq_kernel, P, (const int64_t*)ssm->d_colptr,
                                      (const uint32_t*)ssm->d_vptr, (const int32_t*)ssm->d_idx,
-                                     (const float*)ssm->d_w32, (const float*)rc->d_e32, (const int32_t*)rc->d_start,
+                                     (const float*)ssm->d_w32, (const float*)rc->d_raw, (const int32_t*)rc->d_start,
                                      rc->d_est64, rc->d_x64, cluster, vb));
     CTBB_CUDA(cudaEventRecord(e1, st));
     CTBB_CUDA(cudaEventSynchronize(e1));

@@ -17,9 +17,8 @@
 namespace {
 
 struct FpParams {
-    int nx, ny, nz, nvsm, readings;
+    int nx, ny, nz, nch, nr, nvsm, readings;
     uint64_t nvsm1;
-    SinoLayout lay;
 };
 
 template <class XT>
@@ -45,85 +44,49 @@ __global__ void __launch_bounds__(256) forward_f64_kernel(FpParams P, const int6
         if (v1 <= v0) continue;
         const int64_t cb = colptr[col];
         const int64_t b = cb + vptr[col * P.nvsm1 + v0], e = cb + vptr[col * P.nvsm1 + v1];
-        double* const a = acc + ((int64_t)s << P.lay.shift());
+        const int off = s * P.nch * P.nr;
         for (int64_t m = b + lane; m < e; m += 32) {
             const double w = w32 ? (double)w32[m] : (double)__half2float(w16[m]);
-            atomicAdd(a + (uint32_t)idx[m], xv * w);
+            atomicAdd(acc + (idx[m] + off), xv * w);
         }
     }
 }
 
-// Walk of a sinogram in the device layout beside the raw data: a warp takes 4
-// views x 8 row groups of a channel group, a lane one group (4 consecutive
-// elements at most), so both sides move in 64-byte runs. at() gives the group's
-// first element (SINO_END past the sinogram), raw() the raw index of its element k
-// (-1: padding).
-constexpr uint32_t SINO_END = 0xffffffffu;
-struct SinoWalk {
-    SinoLayout l;
-    int views, vgroups, rgroups;
-    uint64_t units;  // warps' worth of work
-    static SinoWalk make(const SinoLayout& l, uint64_t views) {
-        SinoWalk w;
-        w.l = l;
-        w.views = (int)views;
-        w.vgroups = ((int)l.stride + 3) / 4;
-        w.rgroups = (l.nrb + 7) / 8;
-        w.units = (uint64_t)w.vgroups * l.ncb * w.rgroups;
-        return w;
-    }
-    __device__ __forceinline__ int group() const { return 1 << l.shift(); }
-    __device__ __forceinline__ uint32_t at(uint64_t u, int lane, uint32_t* v, uint32_t* c, uint32_t* r) const {
-        const uint32_t rest = (uint32_t)(u / (uint32_t)rgroups), rg = (uint32_t)(u - (uint64_t)rest * rgroups);
-        const uint32_t vg = rest / (uint32_t)l.ncb, cblk = rest - vg * (uint32_t)l.ncb;
-        const uint32_t rblk = rg * 8 + (lane & 7);
-        *v = vg * 4 + (lane >> 3);
-        if (*v >= l.stride || rblk >= (uint32_t)l.nrb) return SINO_END;
-        *c = cblk << l.cb;
-        *r = rblk << l.rb;
-        return ((cblk * (uint32_t)l.nrb + rblk) * l.stride + *v) << l.shift();
-    }
-    __device__ __forceinline__ int64_t raw(uint32_t v, uint32_t c, uint32_t r, int k) const {
-        c += (uint32_t)(k >> l.rb);
-        r += (uint32_t)(k & l.rb);
-        return v < (uint32_t)views && c < (uint32_t)l.nch && r < (uint32_t)l.nr && k < group()
-                   ? (int64_t)r + (int64_t)l.nr * (c + (int64_t)l.nch * v)
-                   : -1;
-    }
-};
+__global__ void residual_kernel(const float* __restrict__ raw, const double* __restrict__ acc,
+                                float* __restrict__ e32, uint64_t n) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        e32[i] = (float)((double)raw[i] - acc[i]);
+}
 
-// e = y - acc (acc null: e = y) in the device layout, padding zero.
-__global__ void __launch_bounds__(256) residual_kernel(SinoWalk W, const float* __restrict__ raw,
-                                                       const double* __restrict__ acc, float* __restrict__ e32) {
-    const int lane = threadIdx.x & 31, g = W.group();
+// A sinogram from the raw data's order to the second layout (padding zero) or back.
+// A warp takes 4 views x 8 row groups of a channel pair, a lane one group's four
+// elements, so both sides move in 64-byte runs.
+template <bool TO_BULK>
+__global__ void __launch_bounds__(256) arrange_kernel(SinoLayout l, int views, const float* __restrict__ in,
+                                                      float* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t rgroups = ((uint32_t)l.nrb + 7) / 8, vgroups = l.stride / 4;
+    const uint64_t units = (uint64_t)vgroups * (uint32_t)l.ncb * rgroups;
     const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    for (uint64_t u = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); u < W.units; u += nwarps) {
-        uint32_t v = 0, c = 0, r = 0;
-        const uint32_t a = W.at(u, lane, &v, &c, &r);
-        if (a == SINO_END) continue;
-        float y[4], o[4];
+    for (uint64_t u = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); u < units; u += nwarps) {
+        const uint32_t rest = (uint32_t)(u / rgroups), vg = rest / (uint32_t)l.ncb;
+        const uint32_t rblk = ((uint32_t)u - rest * rgroups) * 8 + (lane & 7), v = vg * 4 + (lane >> 3);
+        if (rblk >= (uint32_t)l.nrb) continue;
+        const uint32_t c = (rest - vg * (uint32_t)l.ncb) * 2, r = rblk * 2, a = l.at(v, c, r);
+        __align__(16) float t[4] = {0.f, 0.f, 0.f, 0.f};
+        if (!TO_BULK) *reinterpret_cast<float4*>(t) = *reinterpret_cast<const float4*>(in + a);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int64_t q = W.raw(v, c, r, k);
-            y[k] = q >= 0 ? __ldg(raw + q) : 0.f;
+            const uint32_t ck = c + (k >> 1), rk = r + (k & 1);
+            if (v >= (uint32_t)views || ck >= (uint32_t)l.nch || rk >= (uint32_t)l.nr) continue;
+            const uint64_t q = rk + (uint64_t)l.nr * (ck + (uint64_t)l.nch * v);
+            if (TO_BULK)
+                t[k] = in[q];
+            else
+                out[q] = t[k];
         }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) o[k] = acc && k < g ? (float)((double)y[k] - acc[a + k]) : y[k];
-        if (g == 4) {
-            *reinterpret_cast<float4*>(e32 + a) = make_float4(o[0], o[1], o[2], o[3]);
-        } else {
-            for (int k = 0; k < g; ++k) e32[a + k] = o[k];
-        }
+        if (TO_BULK) *reinterpret_cast<float4*>(out + a) = *reinterpret_cast<const float4*>(t);
     }
-}
-
-// A sinogram from one layout to another of the same detector (the destination is
-// zeroed first: its padding).
-template <class T>
-__global__ void sino_copy_kernel(SinoLayout from, SinoLayout to, int views, const T* __restrict__ a, T* __restrict__ b) {
-    const uint64_t n = (uint64_t)views * from.nch * from.nr;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        b[to.from_linear((uint32_t)i)] = a[from.from_linear((uint32_t)i)];
 }
 
 __global__ void f64_to_f32_kernel(const double* __restrict__ a, float* __restrict__ b, uint64_t n) {
@@ -171,36 +134,13 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     return t;
 }
 
-// sum (raw - acc)^2, acc in the device layout.
-__global__ void __launch_bounds__(256) sq_diff_kernel(SinoWalk W, const float* __restrict__ raw,
-                                                      const double* __restrict__ acc, double* __restrict__ partials) {
-    __shared__ double sh[8];
-    double s = 0.0;
-    const int lane = threadIdx.x & 31;
-    const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    for (uint64_t u = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); u < W.units; u += nwarps) {
-        uint32_t v = 0, c = 0, r = 0;
-        const uint32_t a = W.at(u, lane, &v, &c, &r);
-        if (a == SINO_END) continue;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int64_t q = W.raw(v, c, r, k);
-            if (q < 0) continue;
-            const double d = (double)__ldg(raw + q) - acc[a + k];
-            s += d * d;
-        }
-    }
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) partials[blockIdx.x] = s;
-}
-
-// sum a^2 (a sinogram's padding holds zeros).
-__global__ void __launch_bounds__(256) sq_sum_kernel(const float* __restrict__ a, uint64_t n,
-                                                     double* __restrict__ partials) {
+// sum (raw - acc)^2 (acc may be null: sum e32^2 with e32 passed as raw).
+__global__ void __launch_bounds__(256) sq_sum_kernel(const float* __restrict__ a, const double* __restrict__ acc,
+                                                     uint64_t n, double* __restrict__ partials) {
     __shared__ double sh[8];
     double s = 0.0;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const double d = (double)a[i];
+        const double d = acc ? (double)a[i] - acc[i] : (double)a[i];
         s += d * d;
     }
     s = block_sum(s, sh);
@@ -257,18 +197,20 @@ FpParams fp_params(const ctbb_recon* rc, const ctbb_ssm* ssm) {
     P.nx = (int)rc->geom.num_voxels_x;
     P.ny = (int)rc->geom.num_voxels_y;
     P.nz = (int)rc->geom.num_voxels_z;
+    P.nch = (int)rc->geom.n_channels;
+    P.nr = (int)rc->geom.Nrows_projection;
     P.nvsm = (int)ssm->nvsm;
     P.readings = (int)rc->geom.Readings;
     P.nvsm1 = ssm->nvsm + 1;
-    P.lay = rc->lay;
     return P;
 }
 
-// e = y - est (or y alone) in the device layout.
-ctbb_status residual(ctbb_recon* rc, const double* est) {
-    const SinoWalk W = SinoWalk::make(rc->lay, rc->geom.Readings);
-    residual_kernel<<<grid_for(rc->ctx, W.units * 32, 256), 256, 0, rc->ctx->stream>>>(W, rc->d_raw, est, rc->d_e32);
+// e = y - A x (from the FP64 estimate), in the raw data's order.
+ctbb_status residual(ctbb_recon* rc) {
+    residual_kernel<<<grid_for(rc->ctx, rc->data_size, 256), 256, 0, rc->ctx->stream>>>(rc->d_raw, rc->d_est64,
+                                                                                        rc->d_e32, rc->data_size);
     CTBB_CUDA(cudaGetLastError());
+    rc->e_bulk = false;
     return CTBB_OK;
 }
 
@@ -276,67 +218,36 @@ ctbb_status residual(ctbb_recon* rc, const double* est) {
 
 namespace ctbb {
 
-ctbb_status arranged_raw(ctbb_recon* rc) { return residual(rc, nullptr); }
-
-// One layout for a matrix and a reconstruction. Theirs differ where the scan's
-// number of views is not that of the geometry the matrix was built for: the matrix
-// moves to the scan's layout if its own has too few views, then the reconstruction
-// to the matrix's.
-ctbb_status match_layout(ctbb_recon* rc, const ctbb_ssm* ssm) {
-    if (rc->lay == ssm->lay) return CTBB_OK;
-    if (ssm->lay.stride < rc->geom.Readings) {
-        const uint64_t views = std::max<uint64_t>(rc->geom.Readings, ssm->nvsm);
-        CTBB_TRY(ssm_relayout(const_cast<ctbb_ssm*>(ssm),
-                              SinoLayout::make(rc->geom.n_channels, rc->geom.Nrows_projection, views)));
-        if (rc->lay == ssm->lay) return CTBB_OK;
-    }
-    ctbb_ctx* ctx = rc->ctx;
-    cudaStream_t st = ctx->stream;
-    const uint64_t n = ssm->lay.size();
-    float* e = nullptr;
-    double* est = nullptr;
-    CTBB_CUDA(cudaMalloc(&e, n * sizeof(float)));
-    if (cudaMalloc(&est, n * sizeof(double)) != cudaSuccess) {
-        cudaFree(e);
-        cudaGetLastError();
-        return fail(CTBB_ERR_OOM, "sinogram layout change");
-    }
-    const int views = (int)rc->geom.Readings, grid = grid_for(ctx, rc->data_size, 256);
-    cudaError_t err = cudaMemsetAsync(e, 0, n * sizeof(float), st);
-    if (err == cudaSuccess) err = cudaMemsetAsync(est, 0, n * sizeof(double), st);
-    if (err == cudaSuccess) {
-        sino_copy_kernel<<<grid, 256, 0, st>>>(rc->lay, ssm->lay, views, rc->d_e32, e);
-        sino_copy_kernel<<<grid, 256, 0, st>>>(rc->lay, ssm->lay, views, rc->d_est64, est);
-        err = cudaGetLastError();
-    }
-    if (err == cudaSuccess) err = cudaStreamSynchronize(st);
-    if (err != cudaSuccess) {
-        cudaFree(e);
-        cudaFree(est);
-        return fail(CTBB_ERR_CUDA, "sinogram layout change: %s", cudaGetErrorString(err));
-    }
-    cudaFree(rc->d_e32);
-    cudaFree(rc->d_est64);
-    rc->d_e32 = e;
-    rc->d_est64 = est;
-    rc->lay = ssm->lay;
-    rc->sino_size = n;
-    return CTBB_OK;
-}
-
-ctbb_status check_pair(ctbb_recon* rc, const ctbb_ssm* ssm) {
+ctbb_status check_pair(const ctbb_recon* rc, const ctbb_ssm* ssm) {
     const ctbb_geom_c &a = rc->geom, &b = ssm->geom;
     if (a.num_voxels_x != b.num_voxels_x || a.num_voxels_y != b.num_voxels_y || a.n_channels != b.n_channels ||
         a.Nrows_projection != b.Nrows_projection || a.num_views_for_system_matrix != b.num_views_for_system_matrix)
         return fail(CTBB_ERR_INVALID_ARG, "system matrix geometry does not match the reconstruction");
     if (rc->ctx != ssm->ctx) return fail(CTBB_ERR_INVALID_ARG, "matrix and reconstruction use different contexts");
-    CTBB_CUDA(cudaSetDevice(rc->ctx->device));
-    return match_layout(rc, ssm);
+    return CTBB_OK;
+}
+
+// The buffers stay where they are: through the FP64 estimate's, spare in grouped mode.
+ctbb_status arrange_error(ctbb_recon* rc, bool bulk) {
+    if (rc->e_bulk == bulk) return CTBB_OK;
+    const SinoLayout& l = rc->bulk_lay;
+    const int views = (int)rc->geom.Readings, grid = grid_for(rc->ctx, l.size() / 4, 256);
+    cudaStream_t st = rc->ctx->stream;
+    float* tmp = reinterpret_cast<float*>(rc->d_est64);
+    const uint64_t n = bulk ? rc->data_size : l.size();
+    CTBB_CUDA(cudaMemcpyAsync(tmp, rc->d_e32, n * sizeof(float), cudaMemcpyDeviceToDevice, st));
+    if (bulk)
+        arrange_kernel<true><<<grid, 256, 0, st>>>(l, views, tmp, rc->d_e32);
+    else
+        arrange_kernel<false><<<grid, 256, 0, st>>>(l, views, tmp, rc->d_e32);
+    CTBB_CUDA(cudaGetLastError());
+    rc->e_bulk = bulk;
+    return CTBB_OK;
 }
 
 ctbb_status forward_project_f64(ctbb_recon* rc, const ctbb_ssm* ssm, bool from_x32, double* d_out) {
     ctbb_ctx* ctx = rc->ctx;
-    CTBB_CUDA(cudaMemsetAsync(d_out, 0, rc->sino_size * sizeof(double), ctx->stream));
+    CTBB_CUDA(cudaMemsetAsync(d_out, 0, rc->data_size * sizeof(double), ctx->stream));
     const FpParams P = fp_params(rc, ssm);
     const uint64_t nitems = rc->nvox;
     const int grid = grid_for(ctx, nitems * 32, 256, 16);
@@ -355,7 +266,7 @@ ctbb_status recon_to_grouped(ctbb_recon* rc, const ctbb_ssm* ssm) {
     if (rc->rep == 1) return CTBB_OK;
     ctbb_ctx* ctx = rc->ctx;
     f64_to_f32_kernel<<<grid_for(ctx, rc->nvox, 256), 256, 0, ctx->stream>>>(rc->d_x64, rc->d_x32, rc->nvox);
-    CTBB_TRY(residual(rc, rc->d_est64));
+    CTBB_TRY(residual(rc));
     rc->rep = 1;
     return CTBB_OK;
 }
@@ -377,15 +288,15 @@ ctbb_status cost_f64(ctbb_recon* rc, const ctbb_ssm* ssm, bool exact, double* ou
     double data = 0.0, pen = 0.0;
     const bool quad = rc->geom.penalty == CTBB_PENALTY_QUADRATIC;
     if (rc->rep == 0) {
-        sq_diff_kernel<<<nb, 256, 0, ctx->stream>>>(SinoWalk::make(rc->lay, rc->geom.Readings), rc->d_raw, rc->d_est64,
-                                                    ctx->d_partials);
+        sq_sum_kernel<<<nb, 256, 0, ctx->stream>>>(rc->d_raw, rc->d_est64, rc->data_size, ctx->d_partials);
     } else if (exact) {
         // Recompute A x in FP64 into the (grouped-mode spare) FP64 buffer.
         CTBB_TRY(forward_project_f64(rc, ssm, true, rc->d_est64));
-        sq_diff_kernel<<<nb, 256, 0, ctx->stream>>>(SinoWalk::make(rc->lay, rc->geom.Readings), rc->d_raw, rc->d_est64,
-                                                    ctx->d_partials);
+        sq_sum_kernel<<<nb, 256, 0, ctx->stream>>>(rc->d_raw, rc->d_est64, rc->data_size, ctx->d_partials);
     } else {
-        sq_sum_kernel<<<nb, 256, 0, ctx->stream>>>(rc->d_e32, rc->sino_size, ctx->d_partials);
+        // (the second layout's padding holds zeros)
+        sq_sum_kernel<<<nb, 256, 0, ctx->stream>>>(rc->d_e32, nullptr, rc->e_bulk ? rc->bulk_lay.size() : rc->data_size,
+                                                   ctx->d_partials);
     }
     CTBB_CUDA(cudaGetLastError());
     CTBB_TRY(reduce_partials(ctx, nb, &data));
@@ -425,9 +336,11 @@ extern "C" ctbb_status ctbb_gpu_recon_create(ctbb_ctx* ctx, const ctbb_geom_c* g
     rc->geom = *geom;
     rc->nvox = geom->num_voxels_x * geom->num_voxels_y * geom->num_voxels_z;
     rc->data_size = geom->Readings * geom->n_channels * geom->Nrows_projection;
-    rc->lay = SinoLayout::make(geom->n_channels, geom->Nrows_projection,
-                               std::max(geom->Readings, geom->num_views_for_system_matrix));
-    rc->sino_size = rc->lay.size();
+    rc->bulk_lay = SinoLayout::grouped(geom->n_channels, geom->Nrows_projection,
+                                       std::max(geom->Readings, geom->num_views_for_system_matrix));
+    // e in either layout; the estimate's buffer also holds e while it is rearranged.
+    const uint64_t e_size = std::max(rc->data_size, rc->bulk_lay.size());
+    const uint64_t est_size = std::max(rc->data_size, (e_size + 1) / 2);
     rc->slice_indices.assign(slice_indices, slice_indices + geom->num_voxels_z);
     std::vector<int32_t> start(geom->num_voxels_z);
     for (uint64_t k = 0; k < geom->num_voxels_z; ++k) {
@@ -437,13 +350,13 @@ extern "C" ctbb_status ctbb_gpu_recon_create(ctbb_ctx* ctx, const ctbb_geom_c* g
     CTBB_CUDA(cudaMalloc(&rc->d_start, start.size() * sizeof(int32_t)));
     CTBB_CUDA(cudaMemcpy(rc->d_start, start.data(), start.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     CTBB_CUDA(cudaMalloc(&rc->d_raw, rc->data_size * sizeof(float)));
-    CTBB_CUDA(cudaMalloc(&rc->d_est64, rc->sino_size * sizeof(double)));
-    CTBB_CUDA(cudaMalloc(&rc->d_e32, rc->sino_size * sizeof(float)));
+    CTBB_CUDA(cudaMalloc(&rc->d_est64, est_size * sizeof(double)));
+    CTBB_CUDA(cudaMalloc(&rc->d_e32, e_size * sizeof(float)));
     CTBB_CUDA(cudaMalloc(&rc->d_x64, rc->nvox * sizeof(double)));
     CTBB_CUDA(cudaMalloc(&rc->d_x32, rc->nvox * sizeof(float)));
     CTBB_CUDA(cudaMemsetAsync(rc->d_raw, 0, rc->data_size * sizeof(float), ctx->stream));
-    CTBB_CUDA(cudaMemsetAsync(rc->d_est64, 0, rc->sino_size * sizeof(double), ctx->stream));
-    CTBB_CUDA(cudaMemsetAsync(rc->d_e32, 0, rc->sino_size * sizeof(float), ctx->stream));
+    CTBB_CUDA(cudaMemsetAsync(rc->d_est64, 0, est_size * sizeof(double), ctx->stream));
+    CTBB_CUDA(cudaMemsetAsync(rc->d_e32, 0, e_size * sizeof(float), ctx->stream));
     CTBB_CUDA(cudaMemsetAsync(rc->d_x64, 0, rc->nvox * sizeof(double), ctx->stream));
     CTBB_CUDA(cudaMemsetAsync(rc->d_x32, 0, rc->nvox * sizeof(float), ctx->stream));
     CTBB_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -522,11 +435,11 @@ extern "C" ctbb_status ctbb_gpu_recon_set_volume_estimate(ctbb_recon* rc, const 
         if (estimate == CTBB_ESTIMATE_FORWARD)
             CTBB_TRY(forward_project_f64(rc, ssm, false, rc->d_est64));
         else  // icd_iteration.cpp:47, 63: the estimate stays zero unless a wFBP start forward-projects it
-            CTBB_CUDA(cudaMemsetAsync(rc->d_est64, 0, rc->sino_size * sizeof(double), st));
+            CTBB_CUDA(cudaMemsetAsync(rc->d_est64, 0, rc->data_size * sizeof(double), st));
     } else {
         CTBB_CUDA(cudaMemsetAsync(rc->d_x32, 0, rc->nvox * sizeof(float), st));
         CTBB_CUDA(cudaMemsetAsync(rc->d_x64, 0, rc->nvox * sizeof(double), st));
-        CTBB_CUDA(cudaMemsetAsync(rc->d_est64, 0, rc->sino_size * sizeof(double), st));
+        CTBB_CUDA(cudaMemsetAsync(rc->d_est64, 0, rc->data_size * sizeof(double), st));
     }
     CTBB_CUDA(cudaStreamSynchronize(st));
     rc->rep = 0;  // grouped mode derives e = y - A x on entry (recon_to_grouped)
@@ -615,7 +528,7 @@ extern "C" ctbb_status ctbb_gpu_recon_refresh_residual(ctbb_recon* rc, const ctb
         CTBB_TRY(forward_project_f64(rc, ssm, false, rc->d_est64));
     } else {
         CTBB_TRY(forward_project_f64(rc, ssm, true, rc->d_est64));
-        CTBB_TRY(residual(rc, rc->d_est64));
+        CTBB_TRY(residual(rc));
     }
     CTBB_CUDA(cudaStreamSynchronize(rc->ctx->stream));
     return CTBB_OK;
@@ -655,7 +568,7 @@ extern "C" ctbb_status ctbb_gpu_recon_iterate(ctbb_recon* rc, const ctbb_ssm* ss
             CTBB_TRY(recon_to_grouped(rc, ssm));
             if (opts->refresh_every > 0 && it > 0 && it % opts->refresh_every == 0) {
                 CTBB_TRY(forward_project_f64(rc, ssm, true, rc->d_est64));
-                CTBB_TRY(residual(rc, rc->d_est64));
+                CTBB_TRY(residual(rc));
             }
             uint64_t items = 0;
             double scattered = 0.0;
@@ -675,7 +588,7 @@ extern "C" ctbb_status ctbb_gpu_recon_iterate(ctbb_recon* rc, const ctbb_ssm* ss
             double c = 0.0;
             CTBB_TRY(cost_f64(rc, ssm, true, &c));
             if (rc->rep == 1) {
-                CTBB_TRY(residual(rc, rc->d_est64));
+                CTBB_TRY(residual(rc));
             }
             s.cost = c;
             if (!isnan(prev_cost)) {

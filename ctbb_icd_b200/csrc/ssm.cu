@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256) ssm_cells_kernel(
     SsmParams P, const ViewTab* __restrict__ vt, const ViewTabF* __restrict__ vtf, const double* __restrict__ chA,
     const double* __restrict__ chB, const float2* __restrict__ chF, const double* __restrict__ rowAp,
     const double* __restrict__ rowN, uint16_t* __restrict__ cnt, const int64_t* __restrict__ colptr,
-    const uint32_t* __restrict__ vptr, SinoLayout lay, int32_t* __restrict__ idx, float* __restrict__ w32,
+    const uint32_t* __restrict__ vptr, int32_t* __restrict__ idx, float* __restrict__ w32,
     __half* __restrict__ w16) {
     // A block walks a column's views: no divisions per cell, and neighbouring
     // lanes meet neighbouring channels and rows.
@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(256) ssm_cells_kernel(
         uint32_t n = 0;
         int64_t base = 0;
         if (FILL) base = colptr[col] + (int64_t)vptr[col * (uint64_t)(P.nvsm + 1) + v];
+        const int q_view = P.nr * P.nch * v;
         float w;
         if (FILL) {
             int ch = ch_lo - 1, r = 0, r_hi = -1;
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(256) ssm_cells_kernel(
                 if (ch > ch_hi) break;
                 if (ray_weight(P, vt[v], chA[ch], chB[ch], rowAp[r], rowN[r], ic, jc, &w)) {
                     const int64_t o = base + n;
-                    idx[o] = (int32_t)lay.at((uint32_t)v, (uint32_t)ch, (uint32_t)r);
+                    idx[o] = r + P.nr * ch + q_view;
                     if (w32) w32[o] = w;
                     if (w16) w16[o] = __float2half_rn(w);
                     ++n;
@@ -317,22 +318,16 @@ __global__ void f32_to_f16_kernel(const float* __restrict__ in, __half* __restri
 // runs of two consecutive sinogram indices. A pair {q, w0 | w1 << 16} holds
 // both FP16 weights of a run in 8 bytes (4 per entry instead of 6); a lone
 // entry has w1 = 0. One thread per (column, view) cell: pair count, then
-// (after the same per-column / per-matrix scans as the entries) the fill.
-// Whether an index and its row successor lie in the same channel (the last row's
-// successor falls into the next channel group).
-__device__ __forceinline__ bool same_channel(const SinoLayout& l, uint32_t a, uint32_t b) {
-    return a / l.plane() == b / l.plane();
-}
-
+// (after the same per-column / per-matrix scans as the entries) the fill. In the
+// second sinogram layout a run stays within a channel: the last row's successor,
+// the next channel's first row, is not its neighbour there.
 template <bool FILL>
 __global__ void __launch_bounds__(256) ssm_pairs_kernel(uint64_t ncol, int nvsm, const int64_t* __restrict__ colptr,
                                                         const uint32_t* __restrict__ vptr,
                                                         const int32_t* __restrict__ idx,
-                                                        const __half* __restrict__ w16, uint16_t* __restrict__ cnt,
-                                                        const int64_t* __restrict__ pcolptr,
-                                                        const uint32_t* __restrict__ pvptr, uint2* __restrict__ pairs,
-                                                        SinoLayout lay, unsigned long long* __restrict__ runs) {
-    unsigned long long n_runs = 0;
+                                                        const __half* __restrict__ w16, SinoLayout lay,
+                                                        uint16_t* __restrict__ cnt, const int64_t* __restrict__ pcolptr,
+                                                        const uint32_t* __restrict__ pvptr, uint2* __restrict__ pairs) {
     const uint64_t ncell = ncol * (uint64_t)nvsm;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < ncell; t += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t col = t / (uint64_t)nvsm;
@@ -343,41 +338,24 @@ __global__ void __launch_bounds__(256) ssm_pairs_kernel(uint64_t ncol, int nvsm,
         if (FILL) out = pairs + pcolptr[col] + pvptr[col * (uint64_t)(nvsm + 1) + v];
         int n = 0;
         for (int64_t m = b; m < en;) {
-            // Two rows of one (view, channel); runs that cross a channel stay apart.
-            const uint32_t a = (uint32_t)idx[m];
-            const uint32_t step = (a & lay.row_mask()) == lay.row_mask() ? lay.row_step() : 1u;
-            const bool two = m + 1 < en && (uint32_t)idx[m + 1] == a + step && same_channel(lay, a, a + step);
+            const uint32_t q = (uint32_t)idx[m];
+            const bool two = m + 1 < en && (uint32_t)idx[m + 1] == q + 1 &&
+                             (lay.stride == 0 || (q + 1) % (uint32_t)lay.nr != 0);
             if (FILL) {
                 const uint32_t lo = __half_as_ushort(w16[m]);
                 const uint32_t hi = two ? __half_as_ushort(w16[m + 1]) : 0u;
-                out[n] = make_uint2((uint32_t)idx[m], lo | (hi << 16));
+                out[n] = make_uint2(lay.stride == 0 ? q : lay.from_raw(q), lo | (hi << 16));
             }
             ++n;
             m += two ? 2 : 1;
         }
-        if (!FILL) {
-            cnt[t] = (uint16_t)n;
-            // Runs of two consecutive sinogram indices, across channels too: the
-            // figure that decides whether pairs pay and is reported.
-            for (int64_t m = b; m < en; ++n_runs)
-                m += m + 1 < en && lay.linear((uint32_t)idx[m + 1]) == lay.linear((uint32_t)idx[m]) + 1 ? 2 : 1;
-        }
-    }
-    if (!FILL) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) n_runs += __shfl_xor_sync(0xffffffffu, n_runs, o);
-        if ((threadIdx.x & 31) == 0 && n_runs) atomicAdd(runs, n_runs);
+        if (!FILL) cnt[t] = (uint16_t)n;
     }
 }
 
-// Sinogram indices from one layout to another (single entries, or the first word
-// of entry pairs).
-__global__ void relayout_kernel(SinoLayout from, SinoLayout to, uint32_t* __restrict__ a, int words, uint64_t n) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t v, c, r;
-        from.split(a[i * words], &v, &c, &r);
-        a[i * words] = to.at(v, c, r);
-    }
+__global__ void ssm_restride_pairs_kernel(SinoLayout from, SinoLayout to, uint2* __restrict__ pairs, uint64_t n) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        pairs[i].x = from.restride(pairs[i].x, to);
 }
 
 void free_pairs(ctbb_ssm* s) {
@@ -510,12 +488,23 @@ ctbb_status ssm_validate_geometry(const ctbb_geom_c& g) {
     return CTBB_OK;
 }
 
-// Build (once) the pair form of an FP16 matrix (ssm_pairs_kernel).
-ctbb_status ssm_build_pairs(ctbb_ssm* s) {
-    if (s->d_pairs || s->pairs_checked) return CTBB_OK;
+// The pair form of an FP16 matrix (ssm_pairs_kernel) with its indices in `lay`.
+// One form is held: another layout's is built from the entries in its place (2.2 ms
+// at 160 x 160 columns), or from the pairs themselves between two strides.
+ctbb_status ssm_build_pairs(ctbb_ssm* s, const SinoLayout& lay) {
+    if (s->pairs_checked && (!s->pairs_pay || (s->d_pairs && s->pair_lay == lay))) return CTBB_OK;
     if (!s->d_w16) return fail(CTBB_ERR_INVALID_ARG, "entry pairs need the matrix's FP16 weights");
     ctbb_ctx* ctx = s->ctx;
     cudaStream_t st = ctx->stream;
+    if (s->d_pairs && !s->pair_lay.is_raw() && !lay.is_raw()) {
+        ssm_restride_pairs_kernel<<<grid_for(ctx, s->npairs, 256), 256, 0, st>>>(s->pair_lay, lay, s->d_pairs,
+                                                                                 s->npairs);
+        CTBB_CUDA(cudaGetLastError());
+        s->pair_lay = lay;
+        s->pairs_id += 1;
+        return CTBB_OK;
+    }
+    free_pairs(s);
     const uint64_t ncell = s->ncol * s->nvsm;
     uint16_t* d_cnt = nullptr;
     uint64_t* d_tot = nullptr;
@@ -526,20 +515,10 @@ ctbb_status ssm_build_pairs(ctbb_ssm* s) {
             for (void* q : p) cudaFree(q);
         }
     } tmp;
-    ctbb_status rc = CTBB_OK;
-    auto run = [&]() -> ctbb_status {
-        CTBB_CUDA(cudaMalloc(&d_cnt, std::max<uint64_t>(1, ncell) * sizeof(uint16_t)));
-        tmp.p[0] = d_cnt;
-        CTBB_CUDA(cudaMalloc(&d_tot, std::max<uint64_t>(1, s->ncol) * sizeof(uint64_t)));
-        tmp.p[1] = d_tot;
-        CTBB_CUDA(cudaMalloc(&d_max, 2 * sizeof(unsigned long long)));
-        tmp.p[2] = d_max;
-        CTBB_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(unsigned long long), st));
-        CTBB_CUDA(cudaMalloc(&s->d_pcolptr, (s->ncol + 1) * sizeof(int64_t)));
-        CTBB_CUDA(cudaMalloc(&s->d_pvptr, s->ncol * (s->nvsm + 1) * sizeof(uint32_t)));
-        const int grid = grid_for(ctx, ncell, 256);
+    const int grid = grid_for(ctx, ncell, 256);
+    auto count = [&](const SinoLayout& l, uint64_t* n) -> ctbb_status {
         ssm_pairs_kernel<false><<<grid, 256, 0, st>>>(s->ncol, (int)s->nvsm, s->d_colptr, s->d_vptr, s->d_idx,
-                                                      s->d_w16, d_cnt, nullptr, nullptr, nullptr, s->lay, d_max + 1);
+                                                      s->d_w16, l, d_cnt, nullptr, nullptr, nullptr);
         CTBB_CUDA(cudaGetLastError());
         ssm_column_scan_kernel<<<(int)std::min<uint64_t>(s->ncol, (uint64_t)ctx->sm_count * 32), 256, 0, st>>>(
             d_cnt, (int)s->nvsm, s->ncol, s->d_pvptr, d_tot);
@@ -547,51 +526,51 @@ ctbb_status ssm_build_pairs(ctbb_ssm* s) {
         ssm_colptr_kernel<<<1, 1024, 0, st>>>(d_tot, s->ncol, s->d_pcolptr, d_max);
         CTBB_CUDA(cudaGetLastError());
         int64_t np = 0;
-        unsigned long long runs = 0;
         CTBB_CUDA(cudaMemcpyAsync(&np, s->d_pcolptr + s->ncol, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-        CTBB_CUDA(cudaMemcpyAsync(&runs, d_max + 1, sizeof(runs), cudaMemcpyDeviceToHost, st));
         CTBB_CUDA(cudaStreamSynchronize(st));
-        s->npairs = runs;
-        if (4 * s->npairs > 3 * s->nnz) return CTBB_OK;  // dropped below
-        // Two pairs of padding: the bulk-staged ICD kernel copies whole 16-byte
-        // units and may read one pair past the last.
-        CTBB_CUDA(cudaMalloc(&s->d_pairs, ((uint64_t)np + 2) * sizeof(uint2)));
-        CTBB_CUDA(cudaMemsetAsync(s->d_pairs + np, 0, 2 * sizeof(uint2), st));
-        ssm_pairs_kernel<true><<<grid, 256, 0, st>>>(s->ncol, (int)s->nvsm, s->d_colptr, s->d_vptr, s->d_idx,
-                                                     s->d_w16, nullptr, s->d_pcolptr, s->d_pvptr, s->d_pairs, s->lay,
-                                                     nullptr);
-        CTBB_CUDA(cudaGetLastError());
-        CTBB_CUDA(cudaStreamSynchronize(st));
+        *n = (uint64_t)np;
         return CTBB_OK;
     };
-    rc = run();
-    s->pairs_checked = true;
-    // Pairs pay only where most runs are two rows long (8 bytes per pair
-    // against 6 per entry): with fewer than 4 entries per 3 pairs (the z
-    // flying focal spot splits the runs) the single entries are kept.
-    if (rc != CTBB_OK || 4 * s->npairs > 3 * s->nnz) free_pairs(s);
-    return rc;
-}
-
-// Move the matrix's indices to another layout (a scan with more views than the
-// geometry the matrix was built for).
-ctbb_status ssm_relayout(ctbb_ssm* s, const SinoLayout& to) {
-    if (s->lay == to) return CTBB_OK;
-    cudaStream_t st = s->ctx->stream;
-    if (s->nnz) {
-        relayout_kernel<<<grid_for(s->ctx, s->nnz, 256), 256, 0, st>>>(s->lay, to, (uint32_t*)s->d_idx, 1, s->nnz);
+    bool pay = s->pairs_pay;
+    auto run = [&]() -> ctbb_status {
+        CTBB_CUDA(cudaMalloc(&d_cnt, std::max<uint64_t>(1, ncell) * sizeof(uint16_t)));
+        tmp.p[0] = d_cnt;
+        CTBB_CUDA(cudaMalloc(&d_tot, std::max<uint64_t>(1, s->ncol) * sizeof(uint64_t)));
+        tmp.p[1] = d_tot;
+        CTBB_CUDA(cudaMalloc(&d_max, sizeof(unsigned long long)));
+        tmp.p[2] = d_max;
+        CTBB_CUDA(cudaMemsetAsync(d_max, 0, sizeof(unsigned long long), st));
+        CTBB_CUDA(cudaMalloc(&s->d_pcolptr, (s->ncol + 1) * sizeof(int64_t)));
+        CTBB_CUDA(cudaMalloc(&s->d_pvptr, s->ncol * (s->nvsm + 1) * sizeof(uint32_t)));
+        uint64_t np = 0;
+        if (!s->pairs_checked) {
+            // Pairs pay only where most runs are two rows long (8 bytes per pair
+            // against 6 per entry): with fewer than 4 entries per 3 pairs (the z
+            // flying focal spot splits the runs) the single entries are kept.
+            CTBB_TRY(count(SinoLayout::raw(), &np));
+            pay = 4 * np <= 3 * s->nnz;
+            if (!pay) return CTBB_OK;
+        }
+        if (s->pairs_checked || !lay.is_raw()) CTBB_TRY(count(lay, &np));
+        // Two pairs of padding: the bulk-staged ICD kernel copies whole 16-byte
+        // units and may read one pair past the last.
+        CTBB_CUDA(cudaMalloc(&s->d_pairs, (np + 2) * sizeof(uint2)));
+        CTBB_CUDA(cudaMemsetAsync(s->d_pairs + np, 0, 2 * sizeof(uint2), st));
+        ssm_pairs_kernel<true><<<grid, 256, 0, st>>>(s->ncol, (int)s->nvsm, s->d_colptr, s->d_vptr, s->d_idx,
+                                                     s->d_w16, lay, nullptr, s->d_pcolptr, s->d_pvptr, s->d_pairs);
         CTBB_CUDA(cudaGetLastError());
-    }
-    if (s->d_pairs) {
-        int64_t np = 0;
-        CTBB_CUDA(cudaMemcpyAsync(&np, s->d_pcolptr + s->ncol, sizeof(np), cudaMemcpyDeviceToHost, st));
         CTBB_CUDA(cudaStreamSynchronize(st));
-        relayout_kernel<<<grid_for(s->ctx, (uint64_t)np, 256), 256, 0, st>>>(s->lay, to, (uint32_t*)s->d_pairs, 2,
-                                                                             (uint64_t)np);
-        CTBB_CUDA(cudaGetLastError());
-    }
-    s->lay = to;
-    return CTBB_OK;
+        s->npairs = np;
+        s->pair_lay = lay;
+        s->pairs_id += 1;
+        return CTBB_OK;
+    };
+    const ctbb_status rc = run();
+    if (rc != CTBB_OK || !pay) free_pairs(s);
+    // A first build that fails leaves the single entries; a later one is tried again.
+    if (!s->pairs_checked) s->pairs_pay = rc == CTBB_OK && pay;
+    s->pairs_checked = true;
+    return rc;
 }
 
 }  // namespace ctbb
@@ -690,7 +669,6 @@ extern "C" ctbb_status ctbb_gpu_generate_ssm(ctbb_ctx* ctx, const ctbb_geom_c* g
     s->ctx = ctx;
     ctbb::ctx_retain(ctx);
     s->geom = g;
-    s->lay = SinoLayout::make(g.n_channels, g.Nrows_projection, std::max(g.Readings, g.num_views_for_system_matrix));
     s->ncol = (uint64_t)P.nx * P.ny;
     s->nvsm = (uint64_t)P.nvsm;
     s->ffs = ffs ? 1 : 0;
@@ -721,7 +699,7 @@ extern "C" ctbb_status ctbb_gpu_generate_ssm(ctbb_ctx* ctx, const ctbb_geom_c* g
     CTBB_CUDA(cudaEventRecord(e0, st));
     const int grid = grid_for(ctx, ncell, 256);
     ssm_cells_kernel<false><<<grid, 256, 0, st>>>(P, d_vt, d_vtf, d_A, d_B, d_F, d_ap, d_n, d_cnt, nullptr, nullptr,
-                                                  s->lay, nullptr, nullptr, nullptr);
+                                                  nullptr, nullptr, nullptr);
     CTBB_CUDA(cudaGetLastError());
     ssm_column_scan_kernel<<<(int)std::min<uint64_t>(s->ncol, (uint64_t)ctx->sm_count * 32), 256, 0, st>>>(
         d_cnt, P.nvsm, s->ncol, s->d_vptr, d_tot);
@@ -740,7 +718,7 @@ extern "C" ctbb_status ctbb_gpu_generate_ssm(ctbb_ctx* ctx, const ctbb_geom_c* g
     if (weights & CTBB_SSM_FP32) CTBB_CUDA(cudaMalloc(&s->d_w32, nalloc * sizeof(float)));
     if (weights & CTBB_SSM_FP16) CTBB_CUDA(cudaMalloc(&s->d_w16, nalloc * sizeof(__half)));
     ssm_cells_kernel<true><<<grid, 256, 0, st>>>(P, d_vt, d_vtf, d_A, d_B, d_F, d_ap, d_n, nullptr, s->d_colptr,
-                                                 s->d_vptr, s->lay, s->d_idx, s->d_w32, s->d_w16);
+                                                 s->d_vptr, s->d_idx, s->d_w32, s->d_w16);
     CTBB_CUDA(cudaGetLastError());
     CTBB_CUDA(cudaEventRecord(e1, st));
     CTBB_CUDA(cudaEventSynchronize(e1));
@@ -782,10 +760,7 @@ extern "C" ctbb_status ctbb_gpu_ssm_column(const ctbb_ssm* s, uint64_t column, i
     *nnz = n;
     if (!idx && !w) return CTBB_OK;
     if (cap < n) return fail(CTBB_ERR_INVALID_ARG, "buffer too small");
-    if (idx) {
-        CTBB_CUDA(cudaMemcpy(idx, s->d_idx + cp[0], n * sizeof(int32_t), cudaMemcpyDeviceToHost));
-        for (uint64_t i = 0; i < n; ++i) idx[i] = (int32_t)s->lay.linear((uint32_t)idx[i]);
-    }
+    if (idx) CTBB_CUDA(cudaMemcpy(idx, s->d_idx + cp[0], n * sizeof(int32_t), cudaMemcpyDeviceToHost));
     if (w) {
         if (s->d_w32) {
             CTBB_CUDA(cudaMemcpy(w, s->d_w32 + cp[0], n * sizeof(float), cudaMemcpyDeviceToHost));
@@ -837,8 +812,7 @@ extern "C" ctbb_status ctbb_gpu_ssm_export_reference(const ctbb_ssm* s, const ch
             rec.resize(sizeof(size_t) + cn * 8);
             memcpy(rec.data(), &cnt, sizeof(size_t));
             for (uint64_t i = 0; i < cn; ++i) {
-                const int32_t q = (int32_t)s->lay.linear((uint32_t)hi[cb + i]);
-                memcpy(rec.data() + sizeof(size_t) + i * 8, &q, 4);
+                memcpy(rec.data() + sizeof(size_t) + i * 8, &hi[cb + i], 4);
                 memcpy(rec.data() + sizeof(size_t) + i * 8 + 4, &hw[cb + i], 4);
             }
             if (fwrite(rec.data(), 1, rec.size(), f) != rec.size()) {
@@ -862,8 +836,6 @@ extern "C" ctbb_status ctbb_gpu_ssm_import_reference(ctbb_ctx* ctx, const ctbb_g
     const ctbb_geom_c& g = *geom;
     const uint64_t ncol = g.num_voxels_x * g.num_voxels_y, nvsm = g.num_views_for_system_matrix;
     const uint64_t per_view = g.n_channels * g.Nrows_projection;
-    const SinoLayout lay =
-        SinoLayout::make(g.n_channels, g.Nrows_projection, std::max(g.Readings, g.num_views_for_system_matrix));
     FILE* f = fopen(path, "rb");
     if (!f) return fail(CTBB_ERR_IO, "matrix file not found: %s", path);
     std::vector<int64_t> cp(ncol + 1, 0);
@@ -902,7 +874,7 @@ extern "C" ctbb_status ctbb_gpu_ssm_import_reference(ctbb_ctx* ctx, const ctbb_g
             }
             last = q;
             v[q / per_view + 1] += 1;
-            hi.push_back((int32_t)lay.from_linear((uint32_t)q));
+            hi.push_back(q);
             hw.push_back(w);
         }
         for (uint64_t k = 0; k < nvsm; ++k) v[k + 1] += v[k];
@@ -924,7 +896,6 @@ extern "C" ctbb_status ctbb_gpu_ssm_import_reference(ctbb_ctx* ctx, const ctbb_g
     s->ctx = ctx;
     ctbb::ctx_retain(ctx);
     s->geom = g;
-    s->lay = lay;
     s->ncol = ncol;
     s->nvsm = nvsm;
     s->nnz = (uint64_t)cp[ncol];

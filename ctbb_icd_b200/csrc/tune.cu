@@ -27,6 +27,7 @@ extern "C" ctbb_status ctbb_gpu_recon_autotune(ctbb_recon* rc, const ctbb_ssm* s
         return fail(CTBB_ERR_INVALID_ARG, "requested weight format is not held by the matrix");
     o.weights = wsel;
     CTBB_TRY(check_pair(rc, ssm));
+    CTBB_CUDA(cudaSetDevice(rc->ctx->device));
     CTBB_TRY(recon_to_grouped(rc, ssm));
     CTBB_TRY(ctbb_gpu_recon_refresh_residual(rc, ssm));
     double c0 = 0.0;
@@ -34,14 +35,14 @@ extern "C" ctbb_status ctbb_gpu_recon_autotune(ctbb_recon* rc, const ctbb_ssm* s
     cudaStream_t st = rc->ctx->stream;
     float *d_xs = nullptr, *d_es = nullptr;
     CTBB_CUDA(cudaMalloc(&d_xs, rc->nvox * sizeof(float)));
-    if (cudaMalloc(&d_es, rc->sino_size * sizeof(float)) != cudaSuccess) {
+    if (cudaMalloc(&d_es, rc->data_size * sizeof(float)) != cudaSuccess) {
         cudaFree(d_xs);
         return fail(CTBB_ERR_OOM, "autotune snapshot");
     }
     auto copy = [&](float* dst_x, const float* src_x, float* dst_e, const float* src_e) {
         cudaError_t e = cudaMemcpyAsync(dst_x, src_x, rc->nvox * sizeof(float), cudaMemcpyDeviceToDevice, st);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(dst_e, src_e, rc->sino_size * sizeof(float), cudaMemcpyDeviceToDevice, st);
+            e = cudaMemcpyAsync(dst_e, src_e, rc->data_size * sizeof(float), cudaMemcpyDeviceToDevice, st);
         return e;
     };
     ctbb_status status = CTBB_OK;
@@ -92,7 +93,7 @@ extern "C" ctbb_status ctbb_gpu_recon_autotune(ctbb_recon* rc, const ctbb_ssm* s
     // These kernels read entry pairs only: build them now (outside any
     // stream capture) and skip the kernels for a matrix whose detector-row
     // runs do not pair up (z flying focal spot), which keeps none.
-    if (o.weights == CTBB_SSM_FP16 && status == CTBB_OK) status = ssm_build_pairs(const_cast<ctbb_ssm*>(ssm));
+    if (o.weights == CTBB_SSM_FP16 && status == CTBB_OK) status = ssm_build_pairs(const_cast<ctbb_ssm*>(ssm), SinoLayout::raw());
     if (o.weights == CTBB_SSM_FP16 && status == CTBB_OK && ssm->d_pairs) {
         cands.push_back({8, 4 * sms * 8, 8, 0, 4, 0});
         cands.push_back({8, 3 * sms * 8, 8, 0, 5, 0});
