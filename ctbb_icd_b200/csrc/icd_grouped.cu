@@ -2450,6 +2450,7 @@ struct ctbb_batch {
     uint64_t n_total = 0;
     std::vector<int> merged_T;  // tile edge per scan when d_merged was built
     void* d_scans = nullptr;
+    std::vector<unsigned char> scans;  // what d_scans holds
     cudaGraphExec_t graph = nullptr;
     int graph_warps = 0, graph_weights = 0, graph_stage = 0;
     double graph_relax = 0.0;
@@ -2459,27 +2460,35 @@ namespace {
 
 using namespace ctbb;
 
+// The scans' references as they are now: a reconstruction may have built another
+// visiting order since the last call. The device copy stays where it is, so a
+// captured iteration reads the new ones.
 template <class WT>
 ctbb_status upload_scans(ctbb_batch* b, const ctbb_icd_opts& o) {
-    std::vector<ScanRefs<WT>> h(b->recons.size());
-    for (size_t i = 0; i < h.size(); ++i) {
+    std::vector<unsigned char> bytes(b->recons.size() * sizeof(ScanRefs<WT>), 0);
+    for (size_t i = 0; i < b->recons.size(); ++i) {
         ctbb_recon* rc = b->recons[i];
         const ctbb_ssm* s = b->ssms[i];
-        h[i].P = make_params(rc, s, o);
-        h[i].order = rc->d_order;
-        h[i].colptr = s->d_colptr;
-        h[i].vptr = s->d_vptr;
-        h[i].idx = s->d_idx;
-        h[i].w = std::is_same<WT, __half>::value ? (const WT*)s->d_w16 : (const WT*)s->d_w32;
-        h[i].start = rc->d_start;
-        h[i].e = rc->d_e32;
-        h[i].x = rc->d_x32;
+        ScanRefs<WT> h;
+        memset(&h, 0, sizeof(h));  // compared bytewise
+        const GParams P = make_params(rc, s, o);
+        memcpy(&h.P, &P, sizeof(P));
+        h.order = rc->d_order;
+        h.colptr = s->d_colptr;
+        h.vptr = s->d_vptr;
+        h.idx = s->d_idx;
+        h.w = std::is_same<WT, __half>::value ? (const WT*)s->d_w16 : (const WT*)s->d_w32;
+        h.start = rc->d_start;
+        h.e = rc->d_e32;
+        h.x = rc->d_x32;
+        memcpy(bytes.data() + i * sizeof(h), &h, sizeof(h));
     }
-    cudaFree(b->d_scans);
-    b->d_scans = nullptr;
-    CTBB_CUDA(cudaMalloc(&b->d_scans, h.size() * sizeof(ScanRefs<WT>)));
-    CTBB_CUDA(cudaMemcpyAsync(b->d_scans, h.data(), h.size() * sizeof(ScanRefs<WT>), cudaMemcpyHostToDevice,
-                              b->ctx->stream));
+    static_assert(sizeof(ScanRefs<__half>) == sizeof(ScanRefs<float>), "one buffer for both weight formats");
+    if (b->d_scans && bytes == b->scans) return CTBB_OK;
+    b->scans.clear();
+    if (!b->d_scans) CTBB_CUDA(cudaMalloc(&b->d_scans, bytes.size()));
+    CTBB_CUDA(cudaMemcpyAsync(b->d_scans, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, b->ctx->stream));
+    b->scans = bytes;
     return CTBB_OK;
 }
 
@@ -2649,15 +2658,16 @@ extern "C" ctbb_status ctbb_gpu_batch_iterate(ctbb_batch* b, const ctbb_icd_opts
     }
     const int stage = o.stage_column ? 1 : 0;
     if (stage) warps = std::min(warps, b->ctx->sm_count * 4);
+    if (wsel == CTBB_SSM_FP16)
+        CTBB_TRY(upload_scans<__half>(b, o));
+    else
+        CTBB_TRY(upload_scans<float>(b, o));
     if (!b->graph || b->graph_warps != warps || b->graph_relax != relax || b->graph_weights != wsel ||
         b->graph_stage != stage) {
-        if (wsel == CTBB_SSM_FP16) {
-            CTBB_TRY(upload_scans<__half>(b, o));
+        if (wsel == CTBB_SSM_FP16)
             CTBB_TRY(capture_iteration<__half>(b, warps, relax, stage));
-        } else {
-            CTBB_TRY(upload_scans<float>(b, o));
+        else
             CTBB_TRY(capture_iteration<float>(b, warps, relax, stage));
-        }
         b->graph_stage = stage;
         b->graph_warps = warps;
         b->graph_relax = relax;
