@@ -147,9 +147,9 @@ __device__ __forceinline__ Chan chan_filter(const SsmParams& P, const ViewTabF& 
     const float last = (float)(P.nr - 1);
     c.r_lo = (int)fmaxf(ceilf(ka - d), 0.f);
     c.r_hi = (int)fminf(floorf(kb + d), last);
-    if (u > lo + P.tol && u < hi - P.tol) {
-        c.s_lo = (int)fmaxf(ceilf(ka + d), 0.f);
-        c.s_hi = (int)fminf(floorf(kb - d), last);
+    if (u > lo + P.tol && u < hi - P.tol && d < last) {  // (no row is certain of a wider or undefined error)
+        c.s_lo = (int)fminf(fmaxf(ceilf(ka + d), 0.f), last + 1.f);
+        c.s_hi = (int)fmaxf(fminf(floorf(kb - d), last), -1.f);
     }
     return c;
 }
@@ -159,14 +159,16 @@ __device__ __forceinline__ Chan chan_filter(const SsmParams& P, const ViewTabF& 
 // candidate ranges hold some 50 rays per cell of which 2 or 3 contribute, so the
 // FP32 filter above decides every ray that is clearly in or out: the fill
 // evaluates only the rays that contribute (it needs their weights) and the few
-// within the FP32 error of a boundary, the count only the latter.
+// within the FP32 error of a boundary, the count only the latter. Both passes give
+// the same number as long as the filter's margins hold; the fill never stores past
+// the count and reports a cell that has another number of entries.
 template <bool FILL>
 __global__ void __launch_bounds__(256) ssm_cells_kernel(
     SsmParams P, const ViewTab* __restrict__ vt, const ViewTabF* __restrict__ vtf, const double* __restrict__ chA,
     const double* __restrict__ chB, const float2* __restrict__ chF, const double* __restrict__ rowAp,
     const double* __restrict__ rowN, uint16_t* __restrict__ cnt, const int64_t* __restrict__ colptr,
     const uint32_t* __restrict__ vptr, int32_t* __restrict__ idx, float* __restrict__ w32,
-    __half* __restrict__ w16) {
+    __half* __restrict__ w16, unsigned long long* __restrict__ differ) {
     // A block walks a column's views: no divisions per cell, and neighbouring
     // lanes meet neighbouring channels and rows.
     const uint64_t ncol = (uint64_t)P.nx * P.ny;
@@ -191,9 +193,13 @@ __global__ void __launch_bounds__(256) ssm_cells_kernel(
         const int pad = P.ffs ? 3 : 1;
         const int ch_lo = max((int)floorf(cmin) - pad, 0);
         const int ch_hi = min((int)ceilf(cmax) + pad, P.nch - 1);
-        uint32_t n = 0;
+        uint32_t n = 0, counted = 0;
         int64_t base = 0;
-        if (FILL) base = colptr[col] + (int64_t)vptr[col * (uint64_t)(P.nvsm + 1) + v];
+        if (FILL) {
+            const uint32_t* vp = vptr + col * (uint64_t)(P.nvsm + 1) + v;
+            base = colptr[col] + (int64_t)vp[0];
+            counted = vp[1] - vp[0];
+        }
         const int q_view = P.nr * P.nch * v;
         float w;
         if (FILL) {
@@ -210,14 +216,17 @@ __global__ void __launch_bounds__(256) ssm_cells_kernel(
                 }
                 if (ch > ch_hi) break;
                 if (ray_weight(P, vt[v], chA[ch], chB[ch], rowAp[r], rowN[r], ic, jc, &w)) {
-                    const int64_t o = base + n;
-                    idx[o] = r + P.nr * ch + q_view;
-                    if (w32) w32[o] = w;
-                    if (w16) w16[o] = __float2half_rn(w);
+                    if (n < counted) {
+                        const int64_t o = base + n;
+                        idx[o] = r + P.nr * ch + q_view;
+                        if (w32) w32[o] = w;
+                        if (w16) w16[o] = __float2half_rn(w);
+                    }
                     ++n;
                 }
                 ++r;
             }
+            if (n != counted) atomicAdd(differ, 1ull);
         } else {
             for (int ch = ch_lo; ch <= ch_hi; ++ch) {
                 const float2 ab = chF[ch];
@@ -627,15 +636,19 @@ extern "C" ctbb_status ctbb_gpu_generate_ssm(ctbb_ctx* ctx, const ctbb_geom_c* g
     P.ivz = (float)(1.0 / g.voxel_size_z);
     // FP32 positions are off by up to four roundings of the lengths they are
     // made of: the source radius and the field of view in-plane, those times the
-    // rays' slope and the source's travel in z. The margins are four times that
-    // and a thousandth of a voxel.
+    // rays' slope, the source's travel in z and the slice's offset. The margins are
+    // four times that and a thousandth of a voxel.
     double zmax = 0.0;
     for (const ViewTab& t : hv) zmax = std::max(zmax, fabs(t.src2));
-    const double reach = 2.0 * (g.focal_spot_radius + g.voxel_size_x * P.nx + g.voxel_size_y * P.ny);
-    const double slope = 2.0 * (fabs(g.center_row) + (double)P.nr) * g.axial_detector_spacing / g.source_detector_distance;
+    double offz = 0.0;
+    for (const ViewTab& t : hv) offz = std::max(offz, fabs(t.off2));
+    const double cx = fabs(P.cvx) + P.nx, cy = fabs(P.cvy) + P.ny;
+    const double reach = 2.0 * (g.focal_spot_radius + g.voxel_size_x * cx + g.voxel_size_y * cy);
+    const double slope = 2.0 * ((fabs(g.center_row) + (double)P.nr) * fabs(g.axial_detector_spacing) + offz) /
+                         g.source_detector_distance;
     const double ulp = 16.0 / 16777216.0;
-    P.tol = (float)(1e-3 + ulp * (reach / std::min(g.voxel_size_x, g.voxel_size_y) + P.nx + P.ny));
-    P.tolz = (float)(1e-3 + ulp * (zmax + reach * slope) / g.voxel_size_z);
+    P.tol = (float)(1e-3 + ulp * (reach / std::min(g.voxel_size_x, g.voxel_size_y) + cx + cy));
+    P.tolz = (float)(1e-3 + ulp * ((zmax + reach * slope) / g.voxel_size_z + fabs(P.cvz)));
 
     Scoped tmp;
     ViewTab* d_vt = nullptr;
@@ -687,9 +700,9 @@ extern "C" ctbb_status ctbb_gpu_generate_ssm(ctbb_ctx* ctx, const ctbb_geom_c* g
     tmp.ptrs.push_back(d_cnt);
     CTBB_CUDA(cudaMalloc(&d_tot, s->ncol * sizeof(uint64_t)));
     tmp.ptrs.push_back(d_tot);
-    CTBB_CUDA(cudaMalloc(&d_max, sizeof(unsigned long long)));
+    CTBB_CUDA(cudaMalloc(&d_max, 2 * sizeof(unsigned long long)));
     tmp.ptrs.push_back(d_max);
-    CTBB_CUDA(cudaMemsetAsync(d_max, 0, sizeof(unsigned long long), st));
+    CTBB_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(unsigned long long), st));
     CTBB_CUDA(cudaMalloc(&s->d_colptr, (s->ncol + 1) * sizeof(int64_t)));
     CTBB_CUDA(cudaMalloc(&s->d_vptr, s->ncol * (s->nvsm + 1) * sizeof(uint32_t)));
 
@@ -699,7 +712,7 @@ extern "C" ctbb_status ctbb_gpu_generate_ssm(ctbb_ctx* ctx, const ctbb_geom_c* g
     CTBB_CUDA(cudaEventRecord(e0, st));
     const int grid = grid_for(ctx, ncell, 256);
     ssm_cells_kernel<false><<<grid, 256, 0, st>>>(P, d_vt, d_vtf, d_A, d_B, d_F, d_ap, d_n, d_cnt, nullptr, nullptr,
-                                                  nullptr, nullptr, nullptr);
+                                                  nullptr, nullptr, nullptr, nullptr);
     CTBB_CUDA(cudaGetLastError());
     ssm_column_scan_kernel<<<(int)std::min<uint64_t>(s->ncol, (uint64_t)ctx->sm_count * 32), 256, 0, st>>>(
         d_cnt, P.nvsm, s->ncol, s->d_vptr, d_tot);
@@ -718,14 +731,18 @@ extern "C" ctbb_status ctbb_gpu_generate_ssm(ctbb_ctx* ctx, const ctbb_geom_c* g
     if (weights & CTBB_SSM_FP32) CTBB_CUDA(cudaMalloc(&s->d_w32, nalloc * sizeof(float)));
     if (weights & CTBB_SSM_FP16) CTBB_CUDA(cudaMalloc(&s->d_w16, nalloc * sizeof(__half)));
     ssm_cells_kernel<true><<<grid, 256, 0, st>>>(P, d_vt, d_vtf, d_A, d_B, d_F, d_ap, d_n, nullptr, s->d_colptr,
-                                                 s->d_vptr, s->d_idx, s->d_w32, s->d_w16);
+                                                 s->d_vptr, s->d_idx, s->d_w32, s->d_w16, d_max + 1);
     CTBB_CUDA(cudaGetLastError());
     CTBB_CUDA(cudaEventRecord(e1, st));
-    CTBB_CUDA(cudaEventSynchronize(e1));
+    unsigned long long differ = 0;
+    CTBB_CUDA(cudaMemcpyAsync(&differ, d_max + 1, sizeof(differ), cudaMemcpyDeviceToHost, st));
+    CTBB_CUDA(cudaStreamSynchronize(st));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    if (differ)
+        return fail(CTBB_ERR_CUDA, "system matrix: %llu cells have another number of entries than counted", differ);
     s->build_ms = ms;
     CTBB_TRY(finish_common(ctx, s, weights));
     guard.s = nullptr;
