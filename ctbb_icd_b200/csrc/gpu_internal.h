@@ -53,10 +53,10 @@ struct ctbb_ctx {
 // neighbouring channels and two rows per view, and its channels drift slowly from
 // view to view, so in the raw data's order (row fastest) neighbouring entries each
 // lie in another 128-byte line. Here a line holds 8 views of a group and a 32-byte
-// sector two: the 16 entry pairs of a warp's load touch 5.3 lines and 13.3 sectors
-// instead of 15.5 and 17 (512 x 512 x 64 benchmark; 6.9 and 10.3 on 2.3 mm voxels;
-// groups of 4 rows of one channel: 5.4 and 13.8, 9.7 and 14.3). A slice's first view
-// still adds a constant to every index of a column. Channels and rows are padded to
+// sector two: the 16 entry pairs of a warp's load touch 5.7 lines and 12.0 sectors
+// instead of 15.0 and 16.4 (mean of 40 columns of the 512 x 512 x 64 benchmark; on
+// 2.3 mm voxels 6.9 and 9.9; groups of 4 rows of one channel: 6.7 and 13.1, 9.7 and
+// 13.7). A slice's first view still adds a constant to every index of a column. Channels and rows are padded to
 // whole groups, views to whole lines; padding holds zeros. stride 0: the raw data's
 // order, also where there is one row or channel or the index would not fit 31 bits.
 struct SinoLayout {

@@ -16,7 +16,7 @@
 // estimate) in registers from the gather to the update, so the update only
 // stores. Left on the critical path: one round trip of estimate loads, one
 // cluster barrier for alpha and beta, the penalty (every CTA evaluates it from the
-// same sums and its own copy of the voxel's neighbours) and one CTA barrier; the
+// same sums and its own copy of the voxel's neighbours) and two CTA barriers; the
 // next voxel's entries are fetched meanwhile. Only the summation order of
 // alpha/beta differs from the reference's OpenMP reduction. Compiled with
 // -fmad=false.

@@ -230,8 +230,12 @@ typedef struct ctbb_ssm_info {
     int32_t weights;        /* CTBB_SSM_* held                             */
     int32_t ffs;            /* 1 if built with a flying focal spot (in-plane and/or z) */
     double build_ms;        /* device time of the last build               */
-    uint64_t n_pairs;       /* entry pairs (0 until a grouped iteration with
-                               entry_pairs has built them)                 */
+    uint64_t n_pairs;       /* entry pairs held (0 until a grouped iteration
+                               with entry_pairs has built them). One form is
+                               held at a time: a full launch of the bulk
+                               kernels (stage_column 4, 6) builds its own,
+                               whose runs end with a channel, in place of
+                               the others' and they theirs                 */
 } ctbb_ssm_info;
 
 /*
