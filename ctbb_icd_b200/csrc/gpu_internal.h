@@ -56,9 +56,10 @@ struct ctbb_ctx {
 // sector two: the 16 entry pairs of a warp's load touch 5.7 lines and 12.0 sectors
 // instead of 15.0 and 16.4 (mean of 40 columns of the 512 x 512 x 64 benchmark; on
 // 2.3 mm voxels 6.9 and 9.9; groups of 4 rows of one channel: 6.7 and 13.1, 9.7 and
-// 13.7). A slice's first view still adds a constant to every index of a column. Channels and rows are padded to
-// whole groups, views to whole lines; padding holds zeros. stride 0: the raw data's
-// order, also where there is one row or channel or the index would not fit 31 bits.
+// 13.7). A slice's first view still adds a constant to every index of a column.
+// Channels and rows are padded to whole groups, views to whole lines; padding holds
+// zeros. stride 0: the raw data's order, also where there is one row or channel or
+// the index would not fit 31 bits.
 struct SinoLayout {
     int nr = 0, nch = 0, nrb = 0, ncb = 0;
     uint32_t stride = 0;  // views, padded
@@ -127,7 +128,7 @@ struct ctbb_ssm {
     bool pairs_checked = false;  // build tried (pairs kept only where they pay)
     bool pairs_pay = false;      // and kept
     SinoLayout pair_lay;         // of the pairs' indices; entries keep the raw data's order
-    uint64_t pairs_id = 0;       // changes with every build of the pairs
+    uint64_t pairs_id = 0;       // changes with the pairs and with their layout
     int weights = 0;
     int ffs = 0;
     double build_ms = 0.0;

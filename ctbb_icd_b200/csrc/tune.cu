@@ -131,6 +131,7 @@ extern "C" ctbb_status ctbb_gpu_recon_autotune(ctbb_recon* rc, const ctbb_ssm* s
                 seen |= tr.wpv == c.warps_per_voxel && tr.w == c.warps_in_flight && tr.t == c.lattice &&
                         tr.epl == c.entries_per_lane && tr.stage == c.stage_column && tr.pairs == c.entry_pairs;
             if (seen) continue;
+            // (e is in the raw data's order here: every trial ends with a refresh)
             if (copy(rc->d_x32, d_xs, rc->d_e32, d_es) != cudaSuccess) {
                 status = fail(CTBB_ERR_CUDA, "autotune restore");
                 break;
